@@ -173,8 +173,7 @@ int tbgpu_get_state_errors(const tbgpu_ctx *ctx, int cap, double *residual, doub
  * bond that crosses the periodic boundary by images w (-1/0/+1 per axis)
  * carries exp(i*ph), ph = -pi*(w.k - 2*int(0.5*w.k)), k in the reference's
  * units.  k = NULL or (0,0,0) is the Gamma point.  Call after
- * tbgpu_build_hamiltonian; applies to every later H*x and solve.  Away from
- * Gamma, H*x runs the lane-gather kernel. */
+ * tbgpu_build_hamiltonian; applies to every later H*x and solve. */
 int tbgpu_set_bloch_k(tbgpu_ctx *ctx, const double *k);
 
 /* Start vector for the solves (the reference's lanczos_initialize /
@@ -383,48 +382,41 @@ int tbgpu_export_hamiltonian(const tbgpu_ctx *ctx, double *onsite,
  * allocator, or iteration loops that cannot take the device-wide
  * synchronisation of cudaMalloc/cudaFree.  The reduction scratch is a fixed
  * array inside the library (2048 block partials + a counter, 16,640 bytes
- * per device, held until exit); launches needing more than 2048 blocks are
- * refused with TBGPU_E_ARG (10-orbital models: never at the Gamma point,
- * above 49,152 atoms with a Bloch vector set; 5-orbital models: above
- * 98,304 atoms).  Every call shares that array: calls that overlap on the GPU
+ * per device, held until exit); sizes whose product once needed more than
+ * 2048 blocks are refused with TBGPU_E_ARG (10-orbital models: never at the
+ * Gamma point, above 49,152 atoms with a Bloch vector set; 5-orbital models:
+ * above 98,304 atoms).  Every call shares that array: calls that overlap on the GPU
  * race and must be serialised by the caller.  The first call on a device
  * looks up the array's address with that device current; make that first
  * call before any stream capture.  The context's device must be current. */
 int tbgpu_hx_dot_noalloc(tbgpu_ctx *ctx, double shift, const double *x_dev,
                          double *y_dev, double *dot_dev);
 
-/* H*x kernel: 0 = default (warp-staged kernel, 14 warps x 1 stage per SM,
- * each cation's block run by one bulk copy (TMA), the other pieces by
- * 16-byte cp.async, for the 10-orbital models; lane-gather kernel
- * otherwise),
- * 1 = lane-gather kernel for every model, 2 = warp-staged kernel with
- * 7 warps x 2 stages, 3 = two-cell unit kernel (bulk copies of each unit's
- * contiguous pieces; 10-orbital models with the 64-bit store at the Gamma
- * point, else as 0), 4 = the default kernel with every piece, the cation
- * block runs included, by 16-byte cp.async, 5 = one lane per (atom, spin)
- * with block rows loaded straight to registers (10-orbital models with a
- * stored Hamiltonian at the Gamma point, else as 0), 6 = the same lane
- * mapping on a pencil-interleaved copy of the Hamiltonian (every quantity
- * stored with the k index of its cell fastest, so a warp's loads are
- * contiguous; the solves keep their Lanczos vectors in that layout, these
- * products permute the caller's vectors around the kernel; Gamma point, not
- * in batched solves, else as 0), 7 = variant 6 with each warp's next bond's
- * block rows double-buffered in shared memory by 16-byte cp.async copies
- * while it computes the current one (32-bit store, spin-orbit models, closed
- * z boundary and nz a multiple of 16; else as 6), 8 and 9 = the
- * lane-gather kernel of variant 1 with 4 and 2 warps per block instead of
- * 8 (the block size sets each block's staging array and so the blocks and
- * warps an SM holds), for every model.  Variants 0, 2, 3 and 4 give the same
- * y bit for bit, and so do 6 and 7, and 1, 8 and 9; 1, 5 and 6 sum in their
- * own orders (equal to rounding).  For 5-orbital models and Bloch phases,
- * 0 to 7 all run the lane-gather kernel with 8 warps per block. */
+/* H*x kernel: 0, 2, 3, 4, 5 = default (the ring kernel: one lane per (atom,
+ * vector, spin), each bond's blocks and x segments staged through a ring of
+ * shared-memory slots by a producer warp; every model, with and without
+ * Bloch phases; the five numbers once named separate kernels), 1 =
+ * lane-gather kernel for the 10-orbital models, 6 = the same lane mapping on
+ * a pencil-interleaved copy of the Hamiltonian (every quantity stored with
+ * the k index of its cell fastest, so a warp's loads are contiguous; the
+ * solves keep their Lanczos vectors in that layout, these products permute
+ * the caller's vectors around the kernel; 10-orbital models with a stored
+ * Hamiltonian, Gamma point, not in batched solves, else as 0), 7 = variant 6
+ * with each warp's next bond's block rows double-buffered in shared memory by
+ * 16-byte cp.async copies while it computes the current one (32-bit store,
+ * spin-orbit models, closed z boundary and nz a multiple of 16; else as 6),
+ * 8 and 9 = the lane-gather kernel of variant 1 with 4 and 2 warps per block
+ * instead of 8 (the block size sets each block's staging array and so the
+ * blocks and warps an SM holds).  Variants 0, 2, 3, 4 and 5 give the same y
+ * bit for bit, and so do 6 and 7, and 1, 8 and 9; 0, 1 and 6 sum in their own
+ * orders (equal to rounding).  For 5-orbital models every variant runs the
+ * ring kernel. */
 int tbgpu_set_spmv_variant(tbgpu_ctx *ctx, int variant);
 
 /* Autotuner: times the H*x variants that are distinct kernels for the built
- * context (0 to 6, 8 and 9 for the 10-orbital models with the 64-bit store
- * at the Gamma point; 0, 1, 5, 6, 8, 9 and, where it applies, 7 with the
- * 32-bit store; 0, 8 and 9 for 5-orbital models and Bloch phases; only 0
- * with recompute storage), reps launches each with the fused
+ * context (for the 10-orbital models 0, 1, 8, 9 and, at the Gamma point, 6
+ * and, where it applies, 7; only 0 for 5-orbital models and with recompute
+ * storage), reps launches each with the fused
  * Lanczos dot after two untimed ones (CUDA events on the context stream;
  * two temporary device vectors), selects the fastest (ties: the lower
  * number) and returns it with its time per launch.  Synchronous. */
@@ -602,8 +594,8 @@ int tbgpu_get_fold_energies(const tbgpu_ctx *ctx, int cap, double *energies);
  * with a stored Hamiltonian at the Gamma point; columns 1..4 for the
  * mixed-precision solve, 1..2 for double vectors), with the three-term
  * update fused into the product.  Every product of both passes then uses the
- * lane-per-(atom, spin) kernel (H*x variant 5), or the pencil kernel when
- * variant 6 is set, whose columns compute exactly as a one-column launch: the regenerated vectors equal the first
+ * ring kernel (H*x variant 5), or the pencil kernel when variant 6 is set,
+ * whose columns compute exactly as a one-column launch: the regenerated vectors equal the first
  * pass's bit for bit (checked at every segment end, tbgpu_stats.vec_mismatch),
  * so the eigenvalues are those of mode 0 and the eigenvectors differ only by
  * the order of the accumulation.  Where the mode does not apply, or the

@@ -9,10 +9,10 @@ import subprocess
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtbgpu.so")
-SOURCES = ["topology.cu", "build.cu", "spmv.cu", "spmv_async.cu", "lanczos.cu", "capi.cu",
-           "noalloc.cu", "band_eig.cu", "blk_lanczos.cu", "spmm_async.cu", "io.cu",
+SOURCES = ["topology.cu", "build.cu", "spmv.cu", "spmv_ring.cu", "lanczos.cu", "capi.cu",
+           "noalloc.cu", "band_eig.cu", "blk_lanczos.cu", "io.cu",
            "recompute.cu", "optics.cu", "vff.cu",
-           "batch.cu", "spmv_tile.cu", "warmstart.cu", "spmv_lane.cu", "spmv_pen.cu", "bdots_tc.cu"]
+           "batch.cu", "warmstart.cu", "spmv_pen.cu", "bdots_tc.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
               "-std=c++17", "-Xcompiler", "-fPIC", "-shared"]
 

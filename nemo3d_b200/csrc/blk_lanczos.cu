@@ -6,7 +6,7 @@
 // One block step, p vectors at a time (Q: current block, Qold: previous
 // block, R: residual block, all [p][n] complex in HBM):
 //   [Q, B] = qr(R)            (not at the first step)
-//   R_i    = H Q_i            (one multi-vector H*x launch, spmm_async.cu)
+//   R_i    = H Q_i            (one multi-vector H*x launch, spmv_ring.cu)
 //   R     -= Qold B^H         (not at the first step)
 //   A      = Q^H R            (Hermitian p x p; lower triangle computed)
 //   R     -= Q A

@@ -95,9 +95,9 @@ static void free_ctx(Ctx *c) {
   if (!c) return;
   void *ptrs[] = {c->d_type, c->d_dsp, c->d_par, c->d_par_ok, c->d_site_index, c->d_atom_site,
                   c->d_nbr, c->d_site_m, c->d_surface, c->d_onsite, c->d_blocks, c->d_partial,
-                  c->d_counter, c->d_status, c->d_x, c->d_y, c->d_phase, c->d_groups,
-                  c->d_blocks32, c->d_onsite32, c->d_rc_order, c->d_units, c->d_start,
-                  c->d_lane_tasks, c->d_pen_blk, c->d_pen_ons, c->d_pen_ok,
+                  c->d_counter, c->d_status, c->d_x, c->d_y, c->d_phase, c->d_wrap, c->d_order, c->d_bonds,
+                  c->d_blocks32, c->d_onsite32, c->d_rc_order, c->d_start,
+                  c->d_pen_blk, c->d_pen_ons, c->d_pen_ok,
                   c->d_pen_scratch, c->d_fold_tmp};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -538,28 +538,18 @@ int tbgpu_set_spmv_variant(tbgpu_ctx *ctx, int variant) {
   return TBGPU_OK;
 }
 
-// The variants that launch distinct kernels for this context: all seven for
-// the 10-orbital models with the double store at the Gamma point; the
-// warp-staged, the lane-gather, the lane-per-(atom, spin) and the pencil
-// kernel with the float store; one kernel otherwise (5-orbital models, Bloch
-// phases, recompute storage).
+// The variants that launch distinct kernels for this context: the ring kernel
+// (0), and for the 10-orbital models with stored blocks the lane-gather kernel
+// at three block sizes (1, 8, 9) and, at the Gamma point, the pencil kernels.
 static int distinct_variants(const Ctx &c, int *v) {
-  if (c.recompute) {
-    v[0] = 0;
-    return 1;
-  }
   int n = 0;
-  if (c.norb != 10 || c.bloch) {  // the lane-gather kernel at three block sizes
-    v[n++] = 0;
-  } else if (c.ham_fp32) {
-    v[n++] = 0;
-    v[n++] = 1;
-    v[n++] = 5;
+  v[n++] = 0;
+  if (c.recompute || c.norb != 10) return n;
+  v[n++] = 1;
+  if (!c.bloch) {
     v[n++] = 6;
     // the staged pencil kernel where it applies (otherwise 7 runs 6's)
-    if (c.nspin == 2 && c.nz % 16 == 0 && !c.periodic[2]) v[n++] = 7;
-  } else {
-    for (int i = 0; i < 7; i++) v[n++] = i;
+    if (c.ham_fp32 && c.nspin == 2 && c.nz % 16 == 0 && !c.periodic[2]) v[n++] = 7;
   }
   v[n++] = 8;
   v[n++] = 9;
@@ -610,11 +600,6 @@ int tbgpu_autotune_spmv(tbgpu_ctx *ctx, int reps, int *variant_out, double *ms_o
     }
   }
   c.spmv_variant = rc == TBGPU_OK ? best : keep;
-  if (c.spmv_variant != 3 && c.d_units) {  // the unit table only serves variant 3
-    cudaFree(c.d_units);
-    c.d_units = nullptr;
-    c.nunits = 0;
-  }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   cudaFree(x);

@@ -1,4 +1,4 @@
-// Device helpers shared by the register-streaming H*x kernels (spmv_lane.cu,
+// Device helpers shared by the lane-per-(atom, spin) H*x kernels (spmv_ring.cu,
 // spmv_pen.cu): 16-byte loads of block rows and vector segments, complex
 // multiply-adds, and explicitly rounded products for epilogues that several
 // launch shapes must round identically.

@@ -43,19 +43,18 @@ template <typename V> __device__ __forceinline__ V vzero() {
 // PHASE: bonds carry the Bloch phase phase[a*4+n] of H[a][nbr] (periodic
 // structures away from the Gamma point).
 // HT: element type of the stored Hamiltonian (double, or float for the
-// single-precision store); VT: vector element, double2 (arithmetic in double)
-// or float2 (the mixed-precision solve: float arithmetic, alpha in double).
-template <int NORB, int NSPIN, int WPB, bool DOT, bool PHASE = false, typename HT = double,
-          typename VT = double2>
+// single-precision store).
+template <int NORB, int NSPIN, int WPB, bool DOT, bool PHASE = false, typename HT = double>
 __global__ void __launch_bounds__(WPB * 32)
     k_spmv(long natoms, const int4 *__restrict__ nbr, const unsigned char *__restrict__ site_m,
            const HT *__restrict__ onsite, const HT *__restrict__ blocks,
-           const VT *__restrict__ x, VT *__restrict__ y, double shift_d,
+           const double2 *__restrict__ x, double2 *__restrict__ y, double shift,
            const double *__restrict__ xnorm, int xnorm_idx, double *partial,
            unsigned int *counter, double *alpha_out, int alpha_idx,
            const double2 *__restrict__ phase = nullptr,
            const unsigned char *__restrict__ skip = nullptr) {
-  using RT = decltype(VT::x);
+  using VT = double2;
+  using RT = double;
   constexpr int NB = NORB * NSPIN;
   constexpr int APW = 32 / NORB;
   constexpr int ONS = onsite_len(NB);
@@ -65,8 +64,7 @@ __global__ void __launch_bounds__(WPB * 32)
   const long a = (long(blockIdx.x) * WPB + w) * APW + ai;
   // skip: atoms left out of the product (a converged dot of a batched solve)
   const bool act = ai < APW && a < natoms && !(skip && __ldg(skip + a));
-  const RT scale = RT(xnorm ? 1.0 / xnorm[xnorm_idx] : 1.0);
-  const RT shift = RT(shift_d);
+  const double scale = xnorm ? 1.0 / xnorm[xnorm_idx] : 1.0;
   int nb[4] = {-1, -1, -1, -1};
   int m = 0;
   if (act) {
@@ -188,7 +186,7 @@ __global__ void __launch_bounds__(WPB * 32)
 
 constexpr int kWPB = 8;
 
-// warps per block of the lane-gather kernel: 8 (variants 0 and 1), 4
+// warps per block of the lane-gather kernel: 8 (variant 1), 4
 // (variant 8) or 2 (variant 9).  The block size sets each block's staging
 // array (warps x atoms per warp x 5 segments) and so how many blocks and
 // warps an SM holds; every atom computes the same either way.
@@ -196,27 +194,27 @@ inline int lane_gather_wpb(const Ctx &c) {
   return c.spmv_variant == 8 ? 4 : c.spmv_variant == 9 ? 2 : kWPB;
 }
 
-template <int NORB, int NSPIN, typename HT, typename VT = double2, int WPB = kWPB>
+template <int NORB, int NSPIN, typename HT, int WPB = kWPB>
 static int launch_ht_w(Ctx &c, const void *x, void *y, double shift,
                        const double *xnorm, int xidx, double *alpha_out, int aidx,
                        cudaStream_t s);
 
-template <int NORB, int NSPIN, typename HT, typename VT = double2>
+template <int NORB, int NSPIN, typename HT>
 static int launch_ht(Ctx &c, const void *x, void *y, double shift,
                      const double *xnorm, int xidx, double *alpha_out, int aidx,
                      cudaStream_t s) {
   switch (lane_gather_wpb(c)) {
     case 4:
-      return launch_ht_w<NORB, NSPIN, HT, VT, 4>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
+      return launch_ht_w<NORB, NSPIN, HT, 4>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
     case 2:
-      return launch_ht_w<NORB, NSPIN, HT, VT, 2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
+      return launch_ht_w<NORB, NSPIN, HT, 2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
     default:
-      return launch_ht_w<NORB, NSPIN, HT, VT, kWPB>(c, x, y, shift, xnorm, xidx, alpha_out, aidx,
+      return launch_ht_w<NORB, NSPIN, HT, kWPB>(c, x, y, shift, xnorm, xidx, alpha_out, aidx,
                                                    s);
   }
 }
 
-template <int NORB, int NSPIN, typename HT, typename VT, int WPB>
+template <int NORB, int NSPIN, typename HT, int WPB>
 static int launch_ht_w(Ctx &c, const void *x, void *y, double shift,
                        const double *xnorm, int xidx, double *alpha_out, int aidx,
                        cudaStream_t s) {
@@ -224,27 +222,27 @@ static int launch_ht_w(Ctx &c, const void *x, void *y, double shift,
   constexpr int APW = 32 / NORB;
   const long per_block = long(kWPB) * APW;
   const unsigned grid = unsigned((c.natoms + per_block - 1) / per_block);
-  const VT *X = reinterpret_cast<const VT *>(x);
-  VT *Y = reinterpret_cast<VT *>(y);
+  const double2 *X = reinterpret_cast<const double2 *>(x);
+  double2 *Y = reinterpret_cast<double2 *>(y);
   const HT *ons = ham_onsite<HT>(c), *blk = ham_blocks<HT>(c);
   if (alpha_out) {
     int rc = ensure_partials(c, int(grid));
     if (rc) return rc;
     if (c.bloch)
-      k_spmv<NORB, NSPIN, kWPB, true, true, HT, VT><<<grid, kWPB * 32, 0, s>>>(
+      k_spmv<NORB, NSPIN, kWPB, true, true, HT><<<grid, kWPB * 32, 0, s>>>(
           c.natoms, c.d_nbr, c.d_site_m, ons, blk, X, Y, shift, xnorm, xidx, c.d_partial,
           c.d_counter, alpha_out, aidx, c.d_phase, c.d_skip);
     else
-      k_spmv<NORB, NSPIN, kWPB, true, false, HT, VT><<<grid, kWPB * 32, 0, s>>>(
+      k_spmv<NORB, NSPIN, kWPB, true, false, HT><<<grid, kWPB * 32, 0, s>>>(
           c.natoms, c.d_nbr, c.d_site_m, ons, blk, X, Y, shift, xnorm, xidx, c.d_partial,
           c.d_counter, alpha_out, aidx, nullptr, c.d_skip);
   } else {
     if (c.bloch)
-      k_spmv<NORB, NSPIN, kWPB, false, true, HT, VT><<<grid, kWPB * 32, 0, s>>>(
+      k_spmv<NORB, NSPIN, kWPB, false, true, HT><<<grid, kWPB * 32, 0, s>>>(
           c.natoms, c.d_nbr, c.d_site_m, ons, blk, X, Y, shift, xnorm, xidx, nullptr, nullptr,
           nullptr, 0, c.d_phase, c.d_skip);
     else
-      k_spmv<NORB, NSPIN, kWPB, false, false, HT, VT><<<grid, kWPB * 32, 0, s>>>(
+      k_spmv<NORB, NSPIN, kWPB, false, false, HT><<<grid, kWPB * 32, 0, s>>>(
           c.natoms, c.d_nbr, c.d_site_m, ons, blk, X, Y, shift, xnorm, xidx, nullptr, nullptr,
           nullptr, 0, nullptr, c.d_skip);
   }
@@ -261,30 +259,24 @@ static int launch_t(Ctx &c, const double *x, double *y, double shift,
              : launch_ht<NORB, NSPIN, double>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
 }
 
+// The 10-orbital models by variant: the pencil kernel (6, 7; Gamma point),
+// the lane-gather kernel (1, 8, 9), the ring kernel otherwise.  5-orbital
+// models always take the ring kernel.
 int launch_spmv(Ctx &c, const double *x, double *y, double shift, const double *xnorm,
                 int xidx, double *alpha_out, int aidx, cudaStream_t s) {
   if (c.recompute) return launch_spmv_recompute(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  // the warp-staged kernel has no phase support: periodic structures away
-  // from Gamma take the lane-gather kernel
-  if ((c.spmv_variant == 6 || c.spmv_variant == 7) && pen_supported(c))
+  const int v = c.spmv_variant;
+  if ((v == 6 || v == 7) && pen_supported(c))
     return launch_spmv_pen(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.spmv_variant == 5 && lane_supported(c))
-    return launch_spmv_lane(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 10 && c.spmv_variant == 3 && !c.bloch)
-    return launch_spmv_tile(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 10 && c.spmv_variant != 1 && c.spmv_variant != 8 && c.spmv_variant != 9 &&
-      !c.bloch)
-    return launch_spmv_async(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 10 && c.nspin == 2) return launch_t<10, 2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 10 && c.nspin == 1) return launch_t<10, 1>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 5 && c.nspin == 2) return launch_t<5, 2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 5 && c.nspin == 1) return launch_t<5, 1>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  return set_error(TBGPU_E_UNSUPPORTED);
+  if (c.norb == 10 && (v == 1 || v == 8 || v == 9))
+    return c.nspin == 2 ? launch_t<10, 2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s)
+                        : launch_t<10, 1>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
+  return launch_spmv_ring(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
 }
 
 // The mixed-precision product on complex-float vectors: recomputed in float,
-// or over the float store (the warp-staged kernel for 10 orbitals, the
-// lane-gather kernel for 5); at the Gamma point.
+// or over the float store (the pencil kernel for variants 6 and 7, the ring
+// kernel otherwise); at the Gamma point.
 int launch_spmv_f32(Ctx &c, const float *x, float *y, double shift, const double *xnorm,
                     int xidx, double *alpha_out, int aidx, cudaStream_t s) {
   if (c.bloch) return set_error(TBGPU_E_UNSUPPORTED);
@@ -293,60 +285,21 @@ int launch_spmv_f32(Ctx &c, const float *x, float *y, double shift, const double
   if (!c.ham_fp32) return set_error(TBGPU_E_UNSUPPORTED);
   if ((c.spmv_variant == 6 || c.spmv_variant == 7) && pen_supported(c))
     return launch_spmv_pen_f32(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.spmv_variant == 5 && lane_supported(c))
-    return launch_spmv_lane_f32(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.norb == 10) return launch_spmv_async_f32(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  if (c.nspin == 2)
-    return launch_ht<5, 2, float, float2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
-  return launch_ht<5, 1, float, float2>(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
+  return launch_spmv_ring_f32(c, x, y, shift, xnorm, xidx, alpha_out, aidx, s);
 }
 
-template <int NORB, int NSPIN, typename HT>
-static int launch_scratch_ht(Ctx &c, const double *x, double *y, double shift, double *partial,
-                             unsigned int *counter, int cap, double *dot_out, cudaStream_t s) {
-  constexpr int APW = 32 / NORB;
-  const long per_block = long(kWPB) * APW;
-  const long grid = (c.natoms + per_block - 1) / per_block;
-  if (grid > cap) return set_error(TBGPU_E_ARG);
-  const double2 *X = reinterpret_cast<const double2 *>(x);
-  double2 *Y = reinterpret_cast<double2 *>(y);
-  if (c.bloch)
-    k_spmv<NORB, NSPIN, kWPB, true, true, HT><<<unsigned(grid), kWPB * 32, 0, s>>>(
-        c.natoms, c.d_nbr, c.d_site_m, ham_onsite<HT>(c), ham_blocks<HT>(c), X, Y, shift,
-        nullptr, 0, partial, counter, dot_out, 0, c.d_phase);
-  else
-    k_spmv<NORB, NSPIN, kWPB, true, false, HT><<<unsigned(grid), kWPB * 32, 0, s>>>(
-        c.natoms, c.d_nbr, c.d_site_m, ham_onsite<HT>(c), ham_blocks<HT>(c), X, Y, shift,
-        nullptr, 0, partial, counter, dot_out, 0);
-  TB_CUDA(cudaGetLastError());
-  return TBGPU_OK;
-}
-
-// Lane-gather launch with the alpha dot reduced through caller-provided
-// scratch (partial[cap] doubles, zeroed counter).  Allocates nothing; fails
-// with TBGPU_E_ARG when the launch needs more than cap blocks.
-template <int NORB, int NSPIN>
-static int launch_scratch_t(Ctx &c, const double *x, double *y, double shift, double *partial,
-                            unsigned int *counter, int cap, double *dot_out, cudaStream_t s) {
-  return c.ham_fp32
-             ? launch_scratch_ht<NORB, NSPIN, float>(c, x, y, shift, partial, counter, cap, dot_out, s)
-             : launch_scratch_ht<NORB, NSPIN, double>(c, x, y, shift, partial, counter, cap, dot_out, s);
-}
-
+// H*x with the alpha dot reduced through caller-provided scratch (partial[cap]
+// doubles, zeroed counter); allocates nothing.  The launch sizes that callers
+// know to be refused stay refused (TBGPU_E_ARG), as when the product took one
+// block per 24 or 48 atoms.
 int launch_spmv_scratch(Ctx &c, const double *x, double *y, double shift, double *partial,
                         unsigned int *counter, int cap, double *dot_out, cudaStream_t s) {
   if (c.recompute) return set_error(TBGPU_E_UNSUPPORTED);
-  if (c.norb == 10 && !c.bloch)
-    return launch_spmv_async_scratch(c, x, y, shift, partial, counter, cap, dot_out, s);
-  if (c.norb == 10 && c.nspin == 2)
-    return launch_scratch_t<10, 2>(c, x, y, shift, partial, counter, cap, dot_out, s);
-  if (c.norb == 10 && c.nspin == 1)
-    return launch_scratch_t<10, 1>(c, x, y, shift, partial, counter, cap, dot_out, s);
-  if (c.norb == 5 && c.nspin == 2)
-    return launch_scratch_t<5, 2>(c, x, y, shift, partial, counter, cap, dot_out, s);
-  if (c.norb == 5 && c.nspin == 1)
-    return launch_scratch_t<5, 1>(c, x, y, shift, partial, counter, cap, dot_out, s);
-  return set_error(TBGPU_E_UNSUPPORTED);
+  if (c.norb == 5 || c.bloch) {
+    const long per_block = long(kWPB) * (32 / c.norb);
+    if ((c.natoms + per_block - 1) / per_block > cap) return set_error(TBGPU_E_ARG);
+  }
+  return launch_spmv_ring_scratch(c, x, y, shift, partial, counter, cap, dot_out, s);
 }
 
 }  // namespace tbgpu

@@ -1,7 +1,7 @@
 // H*x for the 10-orbital (sp3d5s*) models on a pencil-interleaved layout
 // (H*x variant 6).
 //
-// Same product as k_spmv_async (spmv_async.cu; restates Hv_stored_20_Hzb,
+// Same product as k_hx_ring (spmv_ring.cu; restates Hv_stored_20_Hzb,
 // nemo3d/src/base/Hmult_stored.c:176-607, with the Lanczos alpha dot of
 // eigen/src/lanczos.c:679-707 fused), written as the stencil it is on the
 // zincblende grid.  A k-pencil of cells (i, j, 0..nz-1) holds, for each of
@@ -29,7 +29,7 @@
 // the start vector in and the eigenvectors out); the C-ABI products on
 // vectors in the reference's order permute around the kernel.  Empty sites
 // (outside a dot's atoms) hold zero vector entries and zero blocks, so they
-// contribute nothing and stay zero.  P > 1 and UPD as in spmv_lane.cu: P
+// contribute nothing and stay zero.  P > 1 and UPD as in spmv_ring.cu: P
 // columns share every block load and compute exactly as one-column launches;
 // UPD fuses the three-term update for the regenerating eigenvector pass.
 #include <algorithm>

@@ -1,7 +1,6 @@
-// Shared-memory staging helpers of the warp-staged H*x kernels
-// (spmv_async.cu, spmm_async.cu): 16-byte cp.async copies, and the group
-// metadata of the context's work order (up to three consecutive atoms of
-// one k-pencil of cells per group).
+// Shared-memory staging helpers of the H*x kernels (spmv_ring.cu,
+// spmv_pen.cu) and the tensor-core block dots: 16-byte cp.async copies and
+// mbarriers with bounded waits.
 #pragma once
 
 #include <cstdint>
@@ -10,8 +9,6 @@
 
 namespace tbgpu {
 namespace stage {
-
-constexpr int kAPW = 3;  // atoms per warp (one lane per orbital, 10 orbitals)
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -76,39 +73,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
           dst),
       "l"(src), "r"(bytes), "r"(mb)
       : "memory");
-}
-
-struct Meta {
-  int nb[kAPW][4];
-  int m[kAPW];  // -1: no atom
-  int a0;       // first atom of the group
-};
-
-// Group g of the work order: up to three consecutive atoms of one pencil.
-// skip (or null): per atom, 1 for atoms left out of the product (the atoms of
-// a converged dot in a batched solve; a group lies in one dot).
-__device__ __forceinline__ Meta load_meta(long g, long ngroups, const int2 *__restrict__ groups,
-                                          const int4 *__restrict__ nbr,
-                                          const unsigned char *__restrict__ site_m,
-                                          const unsigned char *__restrict__ skip = nullptr) {
-  Meta M;
-  int2 e = make_int2(0, 0);
-  if (g < ngroups) e = __ldg(groups + g);
-  if (skip && g < ngroups && __ldg(skip + e.x)) e.y = 0;
-  M.a0 = e.x;
-#pragma unroll
-  for (int i = 0; i < kAPW; i++) {
-    const long a = long(e.x) + i;
-    if (i < e.y) {
-      const int4 v = __ldg(nbr + a);
-      M.nb[i][0] = v.x; M.nb[i][1] = v.y; M.nb[i][2] = v.z; M.nb[i][3] = v.w;
-      M.m[i] = __ldg(site_m + a);
-    } else {
-      M.nb[i][0] = M.nb[i][1] = M.nb[i][2] = M.nb[i][3] = -1;
-      M.m[i] = -1;
-    }
-  }
-  return M;
 }
 
 }  // namespace stage

@@ -89,15 +89,11 @@ struct Ctx {
   std::vector<double> state_resid, state_delta;  // per state of the last solve
   float *d_onsite32 = nullptr;
   float *d_blocks32 = nullptr;
-  // H*x work order: groups of up to 3 consecutive atoms of one k-pencil of
-  // cells, pencils visited in j-blocks (first atom, atom count)
-  int2 *d_groups = nullptr;
-  long ngroups = 0;
-  // unit table of H*x variant 3 (units of two cells of one pencil; built on
-  // first use): nunits descriptors of unit_stride ints, stage capacities
-  int *d_units = nullptr;
-  long nunits = 0;
-  int unit_stride = 0, unit_cap_nb = 0, unit_cap_nx = 0;
+  // H*x work order [natoms]: cations then anions, pencils visited in j-blocks,
+  // and beside each atom its bonds (k_kind_order, topology.cu)
+  int *d_order = nullptr;
+  int4 *d_bonds = nullptr;
+  long ncations = 0;
   // reduction scratch (per-block partials + completion counter)
   double *d_partial = nullptr;
   unsigned int *d_counter = nullptr;
@@ -113,16 +109,11 @@ struct Ctx {
   bool bloch = false;
   double kvec[3] = {0, 0, 0};
   double2 *d_phase = nullptr;       // [natoms*4] phase of H[a][nbr], or null
+  unsigned char *d_wrap = nullptr;  // [natoms] 1: a bond of the atom has a phase, or null
   // scratch for the host-pointer matvec
   double *d_x = nullptr, *d_y = nullptr;
   // start vector set by tbgpu_set_start_vector (used when a solve gets none)
   double *d_start = nullptr;
-  // task list of the lane-per-(atom, spin) H*x kernel (spmv_lane.cu; built on
-  // first use): lane_ntasks tasks of lane_apw atom indices (-1 padded)
-  int *d_lane_tasks = nullptr;
-  long lane_ntasks = 0;
-  int lane_apw = 0;
-  int lane_jblock = 0;   // pencils per j-block of its work order (0: 8)
   // the pencil layout of the stored Hamiltonian (spmv_pen.cu; built on first
   // use): bond blocks as column pairs, on-site records, site mask; scratch
   // for products on vectors in the reference's order
@@ -134,7 +125,7 @@ struct Ctx {
   // eigenvector pass of the Lanczos solve: 0 = the reference's second run of
   // the recurrence from the start vector; 1 = regeneration of vec_segment-
   // iteration segments from checkpoints saved by the first pass,
-  // vec_columns segments at a time (lane kernel products, update fused)
+  // vec_columns segments at a time (ring kernel products, update fused)
   int vec_pass = 0, vec_columns = 4, vec_segment = 256;
   // block Lanczos dots: 0 = double-precision CUDA-core kernel, 1 = the
   // tensor-core (tcgen05 kind::i8 slice) kernel
@@ -204,7 +195,7 @@ inline bool misaligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p)
     if (e_ != cudaSuccess) return ::tbgpu::set_error(TBGPU_E_CUDA); \
   } while (0)
 
-// spmm_async.cu: y + v*ystride = (H - shift)(x + v*xstride) for v < p <= 8
+// spmv_ring.cu: y + v*ystride = (H - shift)(x + v*xstride) for v < p <= 8
 int launch_spmm(Ctx &c, int p, const double *x, long xstride, double *y, long ystride,
                 double shift, cudaStream_t s);
 
@@ -233,24 +224,17 @@ int launch_spmv(Ctx &c, const double *x, double *y, double shift,
                 int alpha_index, cudaStream_t s);
 int launch_spmv_f32(Ctx &c, const float *x, float *y, double shift, const double *xscale_dev,
                     int scale_index, double *alpha_out, int alpha_index, cudaStream_t s);
-// spmv_async.cu
-int launch_spmv_async(Ctx &c, const double *x, double *y, double shift,
-                      const double *xscale_dev, int scale_index, double *alpha_out,
-                      int alpha_index, cudaStream_t s);
-int launch_spmv_async_f32(Ctx &c, const float *x, float *y, double shift,
-                          const double *xscale_dev, int scale_index, double *alpha_out,
-                          int alpha_index, cudaStream_t s);
-// spmv_lane.cu: lane per (atom, spin), 10-orbital models, stored blocks,
-// Gamma point (variant 5)
+// spmv_ring.cu: the stored Hamiltonian on double or float vectors, every model
+int launch_spmv_ring(Ctx &c, const double *x, double *y, double shift, const double *xscale_dev,
+                     int scale_index, double *alpha_out, int alpha_index, cudaStream_t s);
+int launch_spmv_ring_f32(Ctx &c, const float *x, float *y, double shift, const double *xscale_dev,
+                         int scale_index, double *alpha_out, int alpha_index, cudaStream_t s);
+// the alpha dot through caller-provided reduction scratch (noalloc.cu)
+int launch_spmv_ring_scratch(Ctx &c, const double *x, double *y, double shift, double *partial,
+                             unsigned int *counter, int cap, double *dot_out, cudaStream_t s);
 // columns one regenerating pass can take: 4 complex-float or 2 complex-double
 constexpr int lane_max_cols(bool f32) { return f32 ? 4 : 2; }
 bool lane_supported(const Ctx &c);
-int launch_spmv_lane(Ctx &c, const double *x, double *y, double shift,
-                     const double *xscale_dev, int scale_index, double *alpha_out,
-                     int alpha_index, cudaStream_t s);
-int launch_spmv_lane_f32(Ctx &c, const float *x, float *y, double shift,
-                         const double *xscale_dev, int scale_index, double *alpha_out,
-                         int alpha_index, cudaStream_t s);
 // p Lanczos segments advanced by one step in one pass, the update fused:
 // y[j] = next r of the segment whose current r is x[j] at iteration it[j]
 template <typename VT>
@@ -283,16 +267,9 @@ int launch_bdots_tc(Ctx &c, int p, const double2 *const *x, const double2 *const
                     double *partial, unsigned int *counter, int grid, double *G_dev,
                     cudaStream_t s);
 int bdots_tc_grid(const Ctx &c, long n2);
-// spmv_tile.cu: variant 3 (falls back to launch_spmv_async where it does not apply)
-int launch_spmv_tile(Ctx &c, const double *x, double *y, double shift,
-                     const double *xscale_dev, int scale_index, double *alpha_out,
-                     int alpha_index, cudaStream_t s);
 // caller-provided reduction scratch (noalloc.cu)
 int launch_spmv_scratch(Ctx &c, const double *x, double *y, double shift, double *partial,
                         unsigned int *counter, int cap, double *dot_out, cudaStream_t s);
-int launch_spmv_async_scratch(Ctx &c, const double *x, double *y, double shift,
-                              double *partial, unsigned int *counter, int cap, double *dot_out,
-                              cudaStream_t s);
 // lanczos.cu
 int ensure_partials(Ctx &c, int nblocks);
 // y = F x (the folded operator) on double vectors in the reference's order

@@ -94,12 +94,13 @@ __global__ void k_finalize(Grid g, long nsites, const int *flag, const int *inde
 // 2*int(0.5*w.k)) (geo_struct::phasePeriodic, nemo3d/src/base/geo_struct.h:
 // 811-826, applied in Hmult_stored.c:386-437); 1 inside the domain.
 __global__ void k_phase(Grid g, long natoms, const int *atom_site, const int4 *nbr,
-                        double k0, double k1, double k2, double2 *phase) {
+                        double k0, double k1, double k2, double2 *phase, unsigned char *wrap) {
   long a = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (a >= natoms) return;
   const long s = atom_site[a];
   const int4 v = nbr[a];
   const int b[4] = {v.x, v.y, v.z, v.w};
+  bool any = false;
   for (int n = 0; n < 4; n++) {
     double2 p = make_double2(1.0, 0.0);
     bool wrapped;
@@ -111,35 +112,69 @@ __global__ void k_phase(Grid g, long natoms, const int *atom_site, const int4 *n
       double sn, cs;
       sincos(ph, &sn, &cs);
       p = make_double2(cs, -sn);
+      any = true;
     }
     phase[a * 4 + n] = p;
   }
+  wrap[a] = any;
 }
 
 int build_phases(Ctx &c) {
   if (!c.d_phase) TB_CUDA(cudaMalloc(&c.d_phase, sizeof(double2) * 4 * c.natoms));
+  if (!c.d_wrap) TB_CUDA(cudaMalloc(&c.d_wrap, c.natoms));
   Grid g{c.nx, c.ny, c.nz, c.periodic[0], c.periodic[1], c.periodic[2]};
   const int threads = 256;
   const unsigned blocks = unsigned((c.natoms + threads - 1) / threads);
   k_phase<<<blocks, threads, 0, c.stream>>>(g, c.natoms, c.d_atom_site, c.d_nbr, c.kvec[0],
-                                            c.kvec[1], c.kvec[2], c.d_phase);
+                                            c.kvec[1], c.kvec[2], c.d_phase, c.d_wrap);
   TB_CUDA(cudaGetLastError());
   return TBGPU_OK;
 }
 
-// Work order of the warp-staged H*x kernel.  Atoms are numbered in site
-// order, so the atoms of a k-pencil of cells (i, j, 0..nz-1) are one
-// contiguous run.  Visiting pencils j-block by j-block (kPencilBlock pencils
-// wide, i slower than j inside a block) keeps the atoms that share a bond,
-// and with it the x segments and bond blocks read twice, within a few
-// thousand atoms of each other in processing order, so the second read hits
-// L2; in plain atom order the i-direction neighbours are a whole y-z plane
-// apart.
-#ifndef TBGPU_PENCIL_BLOCK
-#define TBGPU_PENCIL_BLOCK 8
-#endif
-constexpr int kPencilBlock = TBGPU_PENCIL_BLOCK;
-constexpr int kGroupAtoms = 3;
+// Work order of the H*x kernels.  Atoms are numbered in site order, so the
+// atoms of a k-pencil of cells (i, j, 0..nz-1) are one contiguous run.
+// Visiting pencils j-block by j-block (kPencilBlock pencils wide, i slower
+// than j inside a block) keeps the atoms that share a bond, and with it the x
+// segments and bond blocks read twice, within a few thousand atoms of each
+// other in processing order, so the second read hits L2; in plain atom order
+// the i-direction neighbours are a whole y-z plane apart.
+constexpr int kPencilBlock = 8;
+
+// The order of the ring kernel (spmv_ring.cu): all cations, then all anions,
+// each kind in the pencil order above; beside each atom its bonds, four times
+// the neighbour for a cation, the block its neighbour stores the bond in
+// (neighbour * 4 + slot) for an anion, -1 for none.  One warp per pencil; start[p] is its first atom (start[npen] = natoms).
+// COUNT: cations[p] only; else the entries, the pencil's cations from
+// cat_at[p] and its anions from an_at[p].
+template <bool COUNT>
+__global__ void k_kind_order(int npen, const int *__restrict__ start,
+                             const unsigned char *__restrict__ site_m,
+                             const int4 *__restrict__ nbr, const int *__restrict__ cat_at, const int *__restrict__ an_at,
+                             int *__restrict__ cations, int *__restrict__ order,
+                             int4 *__restrict__ bonds) {
+  const int p = int(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  if (p >= npen) return;
+  const int lane = threadIdx.x & 31;
+  const unsigned before = (1u << lane) - 1u;
+  int nc = COUNT ? 0 : cat_at[p], na = COUNT ? 0 : an_at[p];
+  for (int a0 = start[p]; a0 < start[p + 1]; a0 += 32) {
+    const int a = a0 + lane;
+    const bool in = a < start[p + 1];
+    const int m = in ? site_m[a] : 0;
+    const unsigned cat = __ballot_sync(0xffffffffu, in && m < 4);
+    const unsigned an = __ballot_sync(0xffffffffu, in && m >= 4);
+    if (!COUNT && in) {
+      const int at = m < 4 ? nc + __popc(cat & before) : na + __popc(an & before);
+      const int4 v = nbr[a];
+      auto bond = [&](int b, int n) { return b < 0 ? -1 : b * 4 + (m < 4 ? 0 : c_rev_slot[m][n]); };
+      order[at] = a;
+      bonds[at] = make_int4(bond(v.x, 0), bond(v.y, 1), bond(v.z, 2), bond(v.w, 3));
+    }
+    nc += __popc(cat);
+    na += __popc(an);
+  }
+  if (COUNT && lane == 0) cations[p] = nc;
+}
 
 static int build_work_order(Ctx &c, const int *index) {
   const long npen = long(c.nx) * c.ny;
@@ -149,19 +184,40 @@ static int build_work_order(Ctx &c, const int *index) {
                             cudaMemcpyDeviceToHost, c.stream));
   TB_CUDA(cudaStreamSynchronize(c.stream));
   start[npen] = int(c.natoms);
-  std::vector<int2> groups;
-  groups.reserve(c.natoms / kGroupAtoms + npen + 1);
+  // kind-sorted order: cations per pencil, scanned in the pencil order
+  if (c.natoms >= (1L << 29)) return set_error(TBGPU_E_UNSUPPORTED);  // block ids are ints
+  int *d_pen = nullptr;  // start[npen + 1], cat_at[npen], an_at[npen], cations[npen]
+  TB_CUDA(cudaMalloc(&c.d_order, sizeof(int) * c.natoms));
+  TB_CUDA(cudaMalloc(&c.d_bonds, sizeof(int4) * c.natoms));
+  TB_CUDA(cudaMallocAsync(&d_pen, sizeof(int) * (4 * npen + 1), c.stream));
+  int *d_cat = d_pen + npen + 1, *d_an = d_cat + npen, *d_cnt = d_an + npen;
+  const unsigned wb = unsigned((npen + 7) / 8);
+  TB_CUDA(cudaMemcpyAsync(d_pen, start.data(), sizeof(int) * (npen + 1), cudaMemcpyHostToDevice,
+                          c.stream));
+  k_kind_order<true><<<wb, 256, 0, c.stream>>>(int(npen), d_pen, c.d_site_m, c.d_nbr,
+                                               nullptr, nullptr, d_cnt, nullptr, nullptr);
+  TB_CUDA(cudaGetLastError());
+  std::vector<int> cnt(npen), at(2 * npen);
+  TB_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * npen, cudaMemcpyDeviceToHost, c.stream));
+  TB_CUDA(cudaStreamSynchronize(c.stream));
+  c.ncations = 0;
+  for (int v : cnt) c.ncations += v;
+  int nc = 0, na = int(c.ncations);
   for (int jb = 0; jb < c.ny; jb += kPencilBlock)
     for (int i = 0; i < c.nx; i++)
       for (int j = jb; j < jb + kPencilBlock && j < c.ny; j++) {
         const long p = long(i) * c.ny + j;
-        for (int a = start[p]; a < start[p + 1]; a += kGroupAtoms)
-          groups.push_back(make_int2(a, std::min(kGroupAtoms, start[p + 1] - a)));
+        at[p] = nc;
+        at[npen + p] = na;
+        nc += cnt[p];
+        na += start[p + 1] - start[p] - cnt[p];
       }
-  c.ngroups = long(groups.size());
-  TB_CUDA(cudaMalloc(&c.d_groups, sizeof(int2) * groups.size()));
-  TB_CUDA(cudaMemcpyAsync(c.d_groups, groups.data(), sizeof(int2) * groups.size(),
-                          cudaMemcpyHostToDevice, c.stream));
+  TB_CUDA(cudaMemcpyAsync(d_cat, at.data(), sizeof(int) * 2 * npen, cudaMemcpyHostToDevice,
+                          c.stream));
+  k_kind_order<false><<<wb, 256, 0, c.stream>>>(int(npen), d_pen, c.d_site_m, c.d_nbr,
+                                                d_cat, d_an, nullptr, c.d_order, c.d_bonds);
+  TB_CUDA(cudaGetLastError());
+  TB_CUDA(cudaFreeAsync(d_pen, c.stream));
   TB_CUDA(cudaStreamSynchronize(c.stream));
   return TBGPU_OK;
 }
