@@ -16,26 +16,29 @@
 //    atom load it together (one broadcast address).
 //  * Tasks are run by pairs of warps.  The producer copies the blocks and the
 //    neighbour x segments of one bond n = 0..3 of the task's atoms into a slot
-//    of the pair's ring by 16-byte cp.async: eight lanes move one 128-byte
-//    line of one atom, so a request touches four whole lines.  The consumer
-//    waits on the slot's barrier, multiplies and hands the slot back.  Every
-//    wait is bounded (TBGPU_E_TIMEOUT in the status word; both warps leave
-//    their loops, no copy is left in flight).  The atom pitches are odd
+//    of the pair's ring: the blocks by bulk copies (TMA, one request a block),
+//    the vectors by 16-byte cp.async, eight lanes to a 128-byte line, so that
+//    both units carry half of the staging.  The consumer waits on the slot's
+//    barrier, multiplies and hands the slot back.  Every wait is bounded
+//    (TBGPU_E_TIMEOUT in the status word; both warps leave their loops after
+//    their copies landed or a second bounded wait).  The atom pitches are odd
 //    multiples of 16 bytes, so the row loads have no bank conflicts.
 //  * The task's own segments (and, for the regenerating product, the r before
 //    them) and on-site records arrive in a slot of their own while the bonds
-//    compute; the results take the own segments' place and leave as whole
-//    lines.
+//    compute; the results take the own segments' place and leave by bulk
+//    stores (single vectors) or as whole lines.
 //
-// What bounds it (10 orbitals, spin, double, 1.02M atoms): 150 KB of slots per
-// SM in flight against a loaded round trip of about 3000 cycles, 139 cycles an
-// atom and SM, where HBM alone (2504 bytes at 6.5 TB/s) would take 115 and the
-// consumers alone 98; an atom costs 81 shared-memory wavefronts.  The kernels
-// it replaced: lane per orbital row with x read by broadcast, 201 wavefronts
-// (0.81 against 0.64 ms); lane per (atom, spin) with rows straight from global
-// memory, one tag lookup per lane and load (float, 381k atoms: 0.181 against
-// 0.124 ms); 5-orbital dots, 0.43M atoms: 0.200 against 0.113 ms; block of 8
-// vectors, 66k atoms: 0.296 against 0.197 ms (all in back-to-back passes).
+// What bounds it (10 orbitals, spin, double, 1.02M atoms): about 120 cycles an
+// atom and SM, where HBM alone (2504 bytes at 6.5 TB/s) would take 115 at full
+// clock, the TMA unit 67, the load/store unit 70 and the consumers 98.  Long
+// runs of it sit at the 1000 W power limit (SM clock 1.5 GHz).  With every
+// copy by cp.async the load/store unit carried 140 cycles and was the bound.
+// The kernels this one replaced: lane per orbital row with x read by
+// broadcast, 201 wavefronts an atom (0.81 against 0.53 ms in back-to-back
+// passes); lane per (atom, spin) with rows straight from global memory, one
+// tag lookup per lane and load (float, 381k atoms: 0.181 against 0.118 ms);
+// lane-gather, 5-orbital dots, 0.43M atoms: 0.200 against 0.104 ms; a staged
+// block product of 8 vectors, 66k atoms: 0.296 against 0.183 ms.
 //
 // Every column of a launch computes as a one-vector launch would, operation
 // for operation, so regenerated recurrences are bit-identical to the first
@@ -122,6 +125,13 @@ struct RingShape {
   static constexpr int BPITCH = (BCH | 1) * 16;
   static constexpr int BMASK = BCH == 50 ? 6 : BCH == 25 ? 7 : BCH == 13 ? 3 : 1;
   static constexpr int BPC = cdiv(BCH + BMASK, 8);    // line pieces per block
+  // Atoms of a task whose block comes by a bulk copy, one request of the TMA
+  // unit (about 17 cycles for 800 bytes, 12 for 400, as many for 200); the
+  // rest come by lines through the load/store unit, which also carries the
+  // vectors.  Small blocks of single vectors leave it a quarter (2M-atom
+  // float dot 0.50 against 0.53 ms, 5-orbital dots 104 against 111 us);
+  // 800-byte blocks none (half of them by lines: 0.48 against 0.44 ms, 1.02M).
+  static constexpr int BULK = BLKB >= 800 || P > 1 || APW < 16 ? APW : APW - 4;
   // a vector segment: NSPIN parts of SEG bytes
   static constexpr int SEG = NORB * int(sizeof(VT));
   static constexpr int XB = NSPIN * SEG;
@@ -278,12 +288,13 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
   const int col = (lane % (P * NSPIN)) / NSPIN, sp = lane % NSPIN;  // vector and spin
   unsigned char *wbase = smem + pair * S::pair_bytes(SLOTS);
   unsigned char *own_p = wbase + SLOTS * S::SLOT;
-  // per slot: full (the 32 producer lanes' copies landed), empty (consumed)
+  // per slot: full (the 32 producer lanes' copies and the bulk copies landed),
+  // empty (consumed)
   const uint32_t bars = smem_addr(wbase) + S::pair_bytes(SLOTS) - 16 * SLOTS;
   if (warp < PAIRS && lane == 0) {
 #pragma unroll
     for (int k = 0; k < SLOTS; k++) {
-      mbar_init(bars + 16 * k, 32);
+      mbar_init(bars + 16 * k, 33);
       mbar_init(bars + 16 * k + 8, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -391,6 +402,8 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
             late = true;
             break;
           }
+          if (lane == 0) mbar_expect_tx(full, uint32_t(S::BULK * S::BCH * 16));
+          __syncwarp();
           // bond 0 of the task is consumed, so the task before it has left
           // the own slot: this task's own data, covered by this bond's barrier
           if (n == SLOTS) issue_own();
@@ -404,17 +417,31 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
             // a cation's own block; for a missing bond the (zeroed) one of the atom
             id[u] = cat || v[u] < 0 ? cur.a[u] * 4 + n : v[u];
           }
-          for_lines<APW, S::BPC>(
-              ag,
-              [&](int s, int u) {
-                const uintptr_t src = reinterpret_cast<uintptr_t>(blocks) + long(of_atom(id, s, u)) * S::BLKB;
-                return S::BLKB % 16 ? src & ~uintptr_t(15) : src;
-              },
-              [&](uintptr_t src, int s, int pc) {
+          // the blocks: one bulk copy per atom for the first BULK, the rest by lines
+          {
+            int mine = id[0];
+#pragma unroll
+            for (int u = 1; u < U; u++) mine = sub == u ? id[u] : mine;
+            const int s = DIRECT ? ag + 4 * sub : lane;
+            if (DIRECT ? sub < S::BULK / 4 : lane < S::BULK) {
+              uintptr_t src = reinterpret_cast<uintptr_t>(blocks) + long(mine) * S::BLKB;
+              if (S::BLKB % 16) src &= ~uintptr_t(15);
+              bulk_g2s(dst + s * S::BPITCH, reinterpret_cast<const void *>(src), S::BCH * 16, full);
+            }
+          }
+          if constexpr (S::BULK < APW) {
+#pragma unroll
+            for (int u = S::BULK / 4; u < APW / 4; u++) {
+              const int s = ag + 4 * u;
+              uintptr_t src = reinterpret_cast<uintptr_t>(blocks) + long(of_atom(id, s, u)) * S::BLKB;
+              if (S::BLKB % 16) src &= ~uintptr_t(15);
+#pragma unroll
+              for (int pc = 0; pc < S::BPC; pc++)
                 line_chunk<S::BCH, 16, S::BMASK>(src, sub, pc, [&](int o) {
                   cpa<16, false>(dst + s * S::BPITCH + o, src + o, true);
                 });
-              });
+            }
+          }
           struct Src { uintptr_t p; bool ok; };
           for_lines<APW * P, S::XPC>(
               ag,
@@ -439,6 +466,9 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
       left = left1;
     }
     cp_wait<0>();
+    if (late)  // once more, bounded, for the bulk copies in flight
+      for (uint32_t k = 0; k < SLOTS; k++)
+        mbar_wait(bars + 16 * k, k < slot ? phase_bit ^ 1 : phase_bit);
   } else {
     // ---- consumer --------------------------------------------------------------
     auto orb = [&](int j) { return H == 1 ? j : j < 4 ? 4 * h + j : 8 + h; };
@@ -464,6 +494,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
     int left = lane_skip(la), rotl = lane_rot(la);
     int4 lb = lane_bonds(q);
     const int seg = (al * P + col) * S::XP + sp * S::SP;  // this lane's segment
+    constexpr bool BULK_OUT = P == 1 && S::XP == S::XB;
     while (q < tasks && !late) {
       const bool cat = !(q & 1), run = runs(la, left);
       const int q2 = advance(q1);
@@ -563,6 +594,8 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
                 for (int k = 0; k < NORB; k++) cfma(acc[k], RT(bk[i * NORB + k]), xn[i]);
             }
           }
+          // (bond 0 also hands the own slot on: its results have left)
+          if (BULK_OUT && n == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();  // every lane has read the slot
           if (lane == 0) mbar_arrive(full + 8);
           if (++slot == SLOTS) {
@@ -644,7 +677,25 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
             for (int j = 0; j < NO; j++) w[orb(j)] = acc[j];
           }
         }
-        __syncwarp();
+        if constexpr (BULK_OUT) {
+          // whole segments by bulk stores: one per four atoms that follow one
+          // another in memory, else one per atom
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          const int lead = (al & ~3) * LPA;  // the four atoms' first lane
+          const int a0 = __shfl_sync(0xffffffffu, la, lead);
+          const unsigned in_run = __ballot_sync(0xffffffffu, valid && la == a0 + (al & 3));
+          constexpr unsigned FOUR = 4 * LPA == 32 ? ~0u : (1u << (4 * LPA % 32)) - 1u;
+          const bool whole = APW % 4 == 0 && ((in_run >> lead) & FOUR) == FOUR;
+          if (whole ? lane == lead : valid && lane == al * LPA) {
+            const uintptr_t dst = reinterpret_cast<uintptr_t>(A.y[0]) + long(la) * S::XB;
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                         "r"(smem_addr(own_p) + al * S::XP), "r"(whole ? 4 * S::XB : S::XB)
+                         : "memory");
+          }
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        } else {
+          __syncwarp();
         for_lines<APW * P, S::XPC>(
             ag, [&](int s, int) { return __shfl_sync(0xffffffffu, valid ? la : -1, (s / P) * LPA); },
             [&](int a, int s, int pc) {
@@ -658,6 +709,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
                   *reinterpret_cast<float2 *>(dst + o) = *reinterpret_cast<const float2 *>(src);
               });
             });
+        }
         // (the own slot is free once bond 0 of the next task is arrived on)
       }
       q = q1;
@@ -669,6 +721,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
       rotl = rotl1;
     }
   }
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   if (late && lane == 0 && status) atomicExch(status, TBGPU_E_TIMEOUT);
   if (DOT) grid_reduce<PAIRS * 64>(dot, partial, counter, alpha_out, alpha_idx, false);
 }
@@ -678,14 +731,14 @@ constexpr int kMaxSmem = 227 * 1024;
 // ms at 1.02M atoms, double.
 constexpr int kSlots = 2;
 
-// Warp pairs per SM: as many as shared memory holds, at most eight.  Eight put
-// two consumers and two producers on every scheduler; nine or ten single warps
-// loaded the schedulers unevenly, drifted apart and read 15 % more from DRAM
-// (1.02M atoms: 2.73 against 2.38 GB).
+// Warp pairs per SM: as many as shared memory holds, at most 12; the
+// 10-orbital double products take at most eight, which leaves them the 128
+// registers a thread they need (nine: 0.63 against 0.53 ms at 1.02M atoms,
+// block of 4 at 381k 0.73 against 0.55).
 template <class S>
-constexpr int ring_pairs() {
-  const int w = kMaxSmem / S::pair_bytes(kSlots);
-  return w > 8 ? 8 : w;
+constexpr int ring_pairs(bool wide) {
+  const int w = kMaxSmem / S::pair_bytes(kSlots), most = wide ? 8 : 12;
+  return w > most ? most : w;
 }
 
 struct RingLaunch {
@@ -701,7 +754,7 @@ struct RingLaunch {
 template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool UPD, bool PHASE>
 int run_ring(Ctx &c, const RingCols<VT, P> &A, RingLaunch L, cudaStream_t s) {
   using S = RingShape<NORB, NSPIN, P, HT, VT, UPD>;
-  constexpr int SLOTS = kSlots, PAIRS = ring_pairs<S>();
+  constexpr int SLOTS = kSlots, PAIRS = ring_pairs<S>(NORB == 10 && sizeof(VT) == 16);
   constexpr int smem = PAIRS * S::pair_bytes(SLOTS);
   static_assert(PAIRS >= 1, "a task does not fit shared memory");
   const auto kernel = k_hx_ring<NORB, NSPIN, P, HT, VT, DOT, UPD, PHASE, PAIRS, SLOTS>;
