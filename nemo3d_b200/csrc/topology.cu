@@ -8,9 +8,7 @@
 //   FindSurfaceAtoms (bit 0, isOnSurface) nemo3d/src/base/geo_struct.c:1374-1463
 // Atoms are numbered in site order (cell-major, k fastest, then in-cell site),
 // which is the reference's vector layout.
-#include <algorithm>
-#include <vector>
-
+#include <cub/block/block_scan.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include "tbgpu_internal.cuh"
@@ -143,32 +141,37 @@ constexpr int kPencilBlock = 8;
 // The order of the ring kernel (spmv_ring.cu): all cations, then all anions,
 // each kind in the pencil order above; beside each atom its bonds, four times
 // the neighbour for a cation, the block its neighbour stores the bond in
-// (neighbour * 4 + slot) for an anion, -1 for none.  One warp per pencil; start[p] is its first atom (start[npen] = natoms).
-// COUNT: cations[p] only; else the entries, the pencil's cations from
-// cat_at[p] and its anions from an_at[p].
+// (neighbour * 4 + slot) for an anion, -1 for none.  Built on the device in
+// three launches (the order was built on the host and copied before, two
+// round trips).  first[p * per] is the first atom of pencil p, per sites each
+// (first[npen * per] = natoms).
+
+// cations[p] (COUNT), or the pencil's entries from at[0][p] and at[1][p] (plus
+// the number of cations); one warp per pencil
 template <bool COUNT>
-__global__ void k_kind_order(int npen, const int *__restrict__ start,
+__global__ void k_kind_order(int npen, long per, const int *__restrict__ first,
                              const unsigned char *__restrict__ site_m,
-                             const int4 *__restrict__ nbr, const int *__restrict__ cat_at, const int *__restrict__ an_at,
+                             const int4 *__restrict__ nbr, const int *__restrict__ at,
                              int *__restrict__ cations, int *__restrict__ order,
                              int4 *__restrict__ bonds) {
   const int p = int(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   if (p >= npen) return;
   const int lane = threadIdx.x & 31;
   const unsigned before = (1u << lane) - 1u;
-  int nc = COUNT ? 0 : cat_at[p], na = COUNT ? 0 : an_at[p];
-  for (int a0 = start[p]; a0 < start[p + 1]; a0 += 32) {
+  const int start = first[p * per], end = first[(p + 1) * per];
+  int nc = COUNT ? 0 : at[p], na = COUNT ? 0 : at[npen + p] + at[2 * npen];
+  for (int a0 = start; a0 < end; a0 += 32) {
     const int a = a0 + lane;
-    const bool in = a < start[p + 1];
+    const bool in = a < end;
     const int m = in ? site_m[a] : 0;
     const unsigned cat = __ballot_sync(0xffffffffu, in && m < 4);
     const unsigned an = __ballot_sync(0xffffffffu, in && m >= 4);
     if (!COUNT && in) {
-      const int at = m < 4 ? nc + __popc(cat & before) : na + __popc(an & before);
+      const int to = m < 4 ? nc + __popc(cat & before) : na + __popc(an & before);
       const int4 v = nbr[a];
       auto bond = [&](int b, int n) { return b < 0 ? -1 : b * 4 + (m < 4 ? 0 : c_rev_slot[m][n]); };
-      order[at] = a;
-      bonds[at] = make_int4(bond(v.x, 0), bond(v.y, 1), bond(v.z, 2), bond(v.w, 3));
+      order[to] = a;
+      bonds[to] = make_int4(bond(v.x, 0), bond(v.y, 1), bond(v.z, 2), bond(v.w, 3));
     }
     nc += __popc(cat);
     na += __popc(an);
@@ -176,49 +179,65 @@ __global__ void k_kind_order(int npen, const int *__restrict__ start,
   if (COUNT && lane == 0) cations[p] = nc;
 }
 
-static int build_work_order(Ctx &c, const int *index) {
-  const long npen = long(c.nx) * c.ny;
-  const size_t pitch = size_t(c.nz) * 8 * sizeof(int);
-  std::vector<int> start(npen + 1);
-  TB_CUDA(cudaMemcpy2DAsync(start.data(), sizeof(int), index, pitch, sizeof(int), npen,
-                            cudaMemcpyDeviceToHost, c.stream));
-  TB_CUDA(cudaStreamSynchronize(c.stream));
-  start[npen] = int(c.natoms);
-  // kind-sorted order: cations per pencil, scanned in the pencil order
+// at[0][p], at[1][p]: cations and anions of the pencils visited before p;
+// at[2 npen]: all cations.  One block.
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads)
+    k_kind_scan(int nx, int ny, long per, const int *__restrict__ first,
+                const int *__restrict__ cations, int *__restrict__ at) {
+  using Scan = cub::BlockScan<int, kScanThreads>;
+  __shared__ typename Scan::TempStorage tmp;
+  const int npen = nx * ny, full = ny / kPencilBlock * kPencilBlock;
+  int nc = 0, na = 0;
+  for (int v0 = 0; v0 < npen; v0 += kScanThreads) {
+    const int v = v0 + int(threadIdx.x);
+    int p = 0, cat = 0, an = 0;
+    if (v < npen) {  // the v-th pencil visited: j-blocks, i, j within the block
+      const bool whole = v < full * nx;
+      const int w = whole ? kPencilBlock : ny - full, r = whole ? v % (w * nx) : v - full * nx;
+      const int jb = whole ? v / (w * nx) * kPencilBlock : full;
+      p = r / w * ny + jb + r % w;
+      cat = cations[p];
+      an = first[(p + 1) * per] - first[p * per] - cat;
+    }
+    int c0, a0, ct, t;
+    Scan(tmp).ExclusiveSum(cat, c0, ct);
+    __syncthreads();
+    Scan(tmp).ExclusiveSum(an, a0, t);
+    __syncthreads();
+    if (v < npen) {
+      at[p] = nc + c0;
+      at[npen + p] = na + a0;
+    }
+    nc += ct;
+    na += t;
+  }
+  if (threadIdx.x == 0) at[2 * npen] = nc;
+}
+
+static int build_work_order(Ctx &c, const int *first) {
   if (c.natoms >= (1L << 29)) return set_error(TBGPU_E_UNSUPPORTED);  // block ids are ints
-  int *d_pen = nullptr;  // start[npen + 1], cat_at[npen], an_at[npen], cations[npen]
-  TB_CUDA(cudaMalloc(&c.d_order, sizeof(int) * c.natoms));
-  TB_CUDA(cudaMalloc(&c.d_bonds, sizeof(int4) * c.natoms));
-  TB_CUDA(cudaMallocAsync(&d_pen, sizeof(int) * (4 * npen + 1), c.stream));
-  int *d_cat = d_pen + npen + 1, *d_an = d_cat + npen, *d_cnt = d_an + npen;
+  const int npen = c.nx * c.ny;
+  const long per = long(c.nz) * 8;
+  int *tmp = nullptr;  // at[2 npen + 1], cations[npen]
+  TB_CUDA(cudaMallocAsync(&tmp, sizeof(int) * (3 * size_t(npen) + 1), c.stream));
+  int *cations = tmp + 2 * size_t(npen) + 1;
+  // one allocation: the bonds, then the order
+  TB_CUDA(cudaMalloc(&c.d_bonds, (sizeof(int4) + sizeof(int)) * c.natoms));
+  c.d_order = reinterpret_cast<int *>(c.d_bonds + c.natoms);
   const unsigned wb = unsigned((npen + 7) / 8);
-  TB_CUDA(cudaMemcpyAsync(d_pen, start.data(), sizeof(int) * (npen + 1), cudaMemcpyHostToDevice,
-                          c.stream));
-  k_kind_order<true><<<wb, 256, 0, c.stream>>>(int(npen), d_pen, c.d_site_m, c.d_nbr,
-                                               nullptr, nullptr, d_cnt, nullptr, nullptr);
+  k_kind_order<true><<<wb, 256, 0, c.stream>>>(npen, per, first, c.d_site_m, c.d_nbr, nullptr,
+                                               cations, nullptr, nullptr);
+  k_kind_scan<<<1, kScanThreads, 0, c.stream>>>(c.nx, c.ny, per, first, cations, tmp);
+  k_kind_order<false><<<wb, 256, 0, c.stream>>>(npen, per, first, c.d_site_m, c.d_nbr, tmp,
+                                                nullptr, c.d_order, c.d_bonds);
   TB_CUDA(cudaGetLastError());
-  std::vector<int> cnt(npen), at(2 * npen);
-  TB_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * npen, cudaMemcpyDeviceToHost, c.stream));
-  TB_CUDA(cudaStreamSynchronize(c.stream));
-  c.ncations = 0;
-  for (int v : cnt) c.ncations += v;
-  int nc = 0, na = int(c.ncations);
-  for (int jb = 0; jb < c.ny; jb += kPencilBlock)
-    for (int i = 0; i < c.nx; i++)
-      for (int j = jb; j < jb + kPencilBlock && j < c.ny; j++) {
-        const long p = long(i) * c.ny + j;
-        at[p] = nc;
-        at[npen + p] = na;
-        nc += cnt[p];
-        na += start[p + 1] - start[p] - cnt[p];
-      }
-  TB_CUDA(cudaMemcpyAsync(d_cat, at.data(), sizeof(int) * 2 * npen, cudaMemcpyHostToDevice,
+  int nc = 0;
+  TB_CUDA(cudaMemcpyAsync(&nc, tmp + 2 * size_t(npen), sizeof(int), cudaMemcpyDeviceToHost,
                           c.stream));
-  k_kind_order<false><<<wb, 256, 0, c.stream>>>(int(npen), d_pen, c.d_site_m, c.d_nbr,
-                                                d_cat, d_an, nullptr, c.d_order, c.d_bonds);
-  TB_CUDA(cudaGetLastError());
-  TB_CUDA(cudaFreeAsync(d_pen, c.stream));
+  TB_CUDA(cudaFreeAsync(tmp, c.stream));
   TB_CUDA(cudaStreamSynchronize(c.stream));
+  c.ncations = nc;
   return TBGPU_OK;
 }
 
