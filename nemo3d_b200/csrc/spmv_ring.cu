@@ -494,6 +494,13 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
     int left = lane_skip(la), rotl = lane_rot(la);
     int4 lb = lane_bonds(q);
     const int seg = (al * P + col) * S::XP + sp * S::SP;  // this lane's segment
+    // Double vectors without a split: 40 registers of sums, as many of a whole
+    // x segment and of two block rows leave none to load ahead, so the x
+    // entries are read as they are used and the next ten block elements while
+    // the last ten are multiplied (block of 4 at 381k atoms 0.54 against 0.57
+    // ms, of 8 at 66k 0.177 against 0.188)
+    constexpr bool PIPE = NORB == 10 && H == 1 && sizeof(VT) == 16;
+    static_assert(!(PIPE && PHASE), "block products have no Bloch phases");
     constexpr bool BULK_OUT = P == 1 && S::XP == S::XB;
     while (q < tasks && !late) {
       const bool cat = !(q & 1), run = runs(la, left);
@@ -521,8 +528,9 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
             const int id = cat || w < 0 ? max(la, 0) * 4 + n : w;
             bk += (unsigned(id) * unsigned(S::BLKB) & 15u) / unsigned(sizeof(HT));
           }
-          VT xn[NORB];
-          lds_seg(reinterpret_cast<const VT *>(st + APW * S::BPITCH + seg), xn);
+          const VT *xp = reinterpret_cast<const VT *>(st + APW * S::BPITCH + seg);
+          VT xn[PIPE ? 1 : NORB];
+          if constexpr (!PIPE) lds_seg(xp, xn);
           if (PHASE && rot) {
             const double2 ph = __ldg(phase + long(max(la, 0)) * 4 + n);
 #pragma unroll
@@ -534,7 +542,50 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
           }
           // cation: y_a[i] += sum_k B_n[i][k] x_nb[k]; anion: y_a[k] += sum_i
           // B[i][k] x_nb[i], B the block its cation neighbour stores
-          if constexpr (H == 2) {
+          if constexpr (PIPE) {
+            RT r[2][10];
+            VT xs[2][2];
+            if (cat) {
+              // step (k, half): five rows of a column pair
+              auto load = [&](int t, RT (&b)[10], VT (&x2)[2]) {
+                const int k = t & ~1, i0 = t & 1 ? 5 : 0;
+#pragma unroll
+                for (int j = 0; j < 5; j++) {
+                  RT v[2];
+                  lds_pairs(bk + (i0 + j) * NORB + k, v, 1);
+                  b[2 * j] = v[0];
+                  b[2 * j + 1] = v[1];
+                }
+                if (!(t & 1)) {
+                  x2[0] = xp[k];
+                  x2[1] = xp[k + 1];
+                }
+              };
+              load(0, r[0], xs[0]);
+#pragma unroll
+              for (int t = 0; t < 10; t++) {
+                if (t < 9) load(t + 1, r[(t + 1) & 1], xs[((t + 1) >> 1) & 1]);
+                const VT(&x2)[2] = xs[(t >> 1) & 1];
+                const int i0 = t & 1 ? 5 : 0;
+#pragma unroll
+                for (int j = 0; j < 5; j++) cfma(acc[i0 + j], r[t & 1][2 * j], x2[0]);
+#pragma unroll
+                for (int j = 0; j < 5; j++) cfma(acc[i0 + j], r[t & 1][2 * j + 1], x2[1]);
+              }
+            } else {
+              lds_pairs(bk, r[0], 5);
+              xs[0][0] = xp[0];
+#pragma unroll
+              for (int i = 0; i < NORB; i++) {
+                if (i < NORB - 1) {
+                  lds_pairs(bk + (i + 1) * NORB, r[(i + 1) & 1], 5);
+                  xs[(i + 1) & 1][0] = xp[i + 1];
+                }
+#pragma unroll
+                for (int k = 0; k < NORB; k++) cfma(acc[k], r[i & 1][k], xs[i & 1][0]);
+              }
+            }
+          } else if constexpr (H == 2) {
             if (cat) {
 #pragma unroll
               for (int k = 0; k < NORB; k += 2) {  // two columns of the lane's five rows
