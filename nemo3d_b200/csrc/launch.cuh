@@ -1,0 +1,42 @@
+// Launches whose start overlaps the end of the kernel before them in the
+// stream (programmatic dependent launch).
+//
+// A kernel launched in the ordinary way starts only after the one before it
+// has ended and its writes are visible: 2 to 3 us between two short kernels.
+// launch_overlapped() lets the blocks of the next one start as soon as every
+// block of the one before has exited, and wait_for_previous() holds them until
+// that kernel is complete and its writes are visible.  So a kernel launched
+// this way calls wait_for_previous() in every thread before its first access
+// to global memory (what precedes it is work on its own shared memory only);
+// the order of the stream then holds as before, also along a chain of such
+// kernels, in stream capture, and behind copies, events or kernels launched
+// in the ordinary way, which the launch waits for in full.
+// H*x of 4096 atoms in a row of calls: 8.3 against 5.4 us a call (then bound
+// by the host); of 66k atoms 39.2 against 38.1 us.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace tbgpu {
+
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+void launch_overlapped(void (*kernel)(Params...), unsigned grid, unsigned block,
+                              size_t smem, cudaStream_t s, Args &&...args) {
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);  // (the caller reads cudaGetLastError)
+}
+
+}  // namespace tbgpu

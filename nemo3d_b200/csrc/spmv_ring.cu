@@ -51,6 +51,7 @@
 #include <type_traits>
 
 #include "lane_math.cuh"
+#include "launch.cuh"
 #include "lanczos_step.cuh"
 #include "reduce.cuh"
 #include "stage.cuh"
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  wait_for_previous();
 
   // The tasks in sequence: cations 0, anions 0, cations 1, ...  Round t of the
   // grid takes the next of them for each of its nw warp pairs, and every pair
@@ -822,10 +824,9 @@ int run_ring(Ctx &c, const RingCols<VT, P> &A, RingLaunch L, cudaStream_t s) {
   } else if (DOT && int(grid) > L.cap) {
     return set_error(TBGPU_E_ARG);
   }
-  kernel<<<grid, PAIRS * 64, smem, s>>>(ncat, nan, c.d_order, c.d_bonds, ham_onsite<HT>(c),
-                                        ham_blocks<HT>(c), A, L.bet, L.alpha, L.shift, L.partial,
-                                        L.counter, L.alpha_out, L.aidx, c.d_phase, c.d_wrap,
-                                        c.d_skip, c.d_status);
+  launch_overlapped(kernel, grid, PAIRS * 64, smem, s, ncat, nan, c.d_order, c.d_bonds,
+                    ham_onsite<HT>(c), ham_blocks<HT>(c), A, L.bet, L.alpha, L.shift, L.partial,
+                    L.counter, L.alpha_out, L.aidx, c.d_phase, c.d_wrap, c.d_skip, c.d_status);
   TB_CUDA(cudaGetLastError());
   return TBGPU_OK;
 }

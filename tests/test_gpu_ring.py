@@ -108,3 +108,61 @@ def test_ring_vectors_off_a_line(model, off):
     yo = o.hx(x[off:].cpu().numpy(), 0.1)
     assert np.abs(y[off:off + n2].cpu().numpy() - yo).max() <= 45e-12 * scale
     assert bool((y[:off] == 7.0).all()) and bool((y[off + n2:] == 7.0).all())
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("name", ["1x1x1", "17x9x11"])
+def test_order_of_overlapped_launches(name, captured):
+    """Products whose starts overlap the kernels before them, between copies,
+    elementwise kernels and a second stream's work: bit for bit what the same
+    calls give with a synchronisation after each one."""
+    import torch
+    from nemo3d_b200.tbgpu import Hamiltonian
+    mats = [materials.MATERIALS["GaAs_spds"], materials.MATERIALS["InAs_spds"]]
+    H = Hamiltonian(STRUCTURES[name](), "sp3d5s*_so", mats)
+    x = torch.from_numpy(np.random.default_rng(7).uniform(-1, 1, 2 * H.n)).cuda()
+    bufs = [torch.zeros_like(x) for _ in range(4)]
+    side = torch.cuda.Stream()
+
+    def work(sync):
+        main, wait = torch.cuda.current_stream(), torch.cuda.synchronize if sync else lambda: None
+        a, b, c, d = bufs
+        a.copy_(x); wait()
+        for k in range(6):
+            H.hx_dev(a.data_ptr(), b.data_ptr(), 0.1 * k); wait()   # reads a, writes b
+            H.hx_dev(b.data_ptr(), a.data_ptr(), 0.2); wait()       # reads b, overwrites a
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                c.copy_(a); c.mul_(0.25)
+            H.hx_dev(a.data_ptr(), d.data_ptr(), 0.3); wait()
+            main.wait_stream(side); wait()
+            H.hx_dev(c.data_ptr(), b.data_ptr(), 0.4); wait()       # behind a join
+            b.add_(d); wait()
+            H.hx_dev(b.data_ptr(), a.data_ptr(), 0.5); wait()       # behind another kernel
+            a.mul_(2.0 ** -8); wait()
+
+    H.set_stream(torch.cuda.current_stream().cuda_stream)
+    work(True)
+    want = [t.clone() for t in bufs]
+    assert torch.isfinite(want[0]).all() and want[0].abs().max() > 0
+    for t in bufs:
+        t.zero_()
+    run = torch.cuda.Stream()
+    run.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(run):
+        H.set_stream(run.cuda_stream)
+        if captured:
+            work(False)
+            graph = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph, stream=run):
+                work(False)
+            for t in bufs:
+                t.zero_()
+            graph.replay()
+            graph.replay()
+        else:
+            work(False)
+    torch.cuda.synchronize()
+    for got, w in zip(bufs, want):
+        assert torch.equal(got, w)
