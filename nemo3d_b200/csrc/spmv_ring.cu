@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
     // the last ten are multiplied (block of 4 at 381k atoms 0.54 against 0.57
     // ms, of 8 at 66k 0.177 against 0.188)
     constexpr bool PIPE = NORB == 10 && H == 1 && sizeof(VT) == 16;
-    static_assert(!(PIPE && PHASE), "block products have no Bloch phases");
+    static_assert(!(PHASE && (PIPE || sizeof(VT) == 8)), "Bloch phases: single double vectors");
     constexpr bool BULK_OUT = P == 1 && S::XP == S::XB;
     while (q < tasks && !late) {
       const bool cat = !(q & 1), run = runs(la, left);
@@ -531,8 +531,9 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
             bk += (unsigned(id) * unsigned(S::BLKB) & 15u) / unsigned(sizeof(HT));
           }
           const VT *xp = reinterpret_cast<const VT *>(st + APW * S::BPITCH + seg);
-          VT xn[PIPE ? 1 : NORB];
-          if constexpr (!PIPE) lds_seg(xp, xn);
+          constexpr bool FLOAT = sizeof(VT) == 8;
+          VT xn[PIPE || FLOAT ? 1 : NORB];
+          if constexpr (!PIPE && !FLOAT) lds_seg(xp, xn);
           if (PHASE && rot) {
             const double2 ph = __ldg(phase + long(max(la, 0)) * 4 + n);
 #pragma unroll
@@ -610,31 +611,67 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
                 cfma(acc[4], r4, xn[i]);
               }
             }
-          } else if constexpr (NORB == 10) {
+          } else if constexpr (FLOAT) {
+            // Float sums: each bond's NORB terms by themselves, then added to
+            // the bonds before them.  One chain of 40 terms is 7.8e-8 off the
+            // 64-bit result (127k atoms, sp3d5s*), the sums by bond 6.3e-8.
+            auto rows2 = [&](int i, RT (&r)[2 * NORB]) {
+              if constexpr (NORB == 10) {
+                lds_rows2(bk + i * NORB, r);
+              } else {
+#pragma unroll
+                for (int k = 0; k < 2 * NORB; k++) r[k] = i * NORB + k < NORB * NORB ? RT(bk[i * NORB + k]) : RT(0);
+              }
+            };
+            auto first_term = [](RT m, VT x) { return VT{m * x.x, m * x.y}; };
             if (cat) {
+              VT xv[NORB];
+              lds_seg(xp, xv);
 #pragma unroll
               for (int i = 0; i < NORB; i += 2) {
-                RT r[20];
-                lds_rows2(bk + i * NORB, r);
+                RT r[2 * NORB];
+                rows2(i, r);
+                VT t0 = first_term(r[0], xv[0]), t1 = first_term(r[NORB], xv[0]);
 #pragma unroll
-                for (int k = 0; k < NORB; k++) {
-                  cfma(acc[i], r[k], xn[k]);
-                  cfma(acc[i + 1], r[NORB + k], xn[k]);
+                for (int k = 1; k < NORB; k++) {
+                  cfma(t0, r[k], xv[k]);
+                  cfma(t1, r[NORB + k], xv[k]);
+                }
+                acc[i].x += t0.x;
+                acc[i].y += t0.y;
+                if (i + 1 < NORB) {
+                  acc[i + 1].x += t1.x;
+                  acc[i + 1].y += t1.y;
                 }
               }
             } else {
+              VT t[NORB];
 #pragma unroll
               for (int i = 0; i < NORB; i += 2) {
-                RT r[20];
-                lds_rows2(bk + i * NORB, r);
+                RT r[2 * NORB];
+                rows2(i, r);
+                VT x2[2];
+                if constexpr (NORB == 10) {
+                  lds_seg(xp + i, x2);
+                } else {
+                  x2[0] = xp[i];
+                  if (i + 1 < NORB) x2[1] = xp[i + 1];
+                }
 #pragma unroll
                 for (int k = 0; k < NORB; k++) {
-                  cfma(acc[k], r[k], xn[i]);
-                  cfma(acc[k], r[NORB + k], xn[i + 1]);
+                  if (i == 0) t[k] = first_term(r[k], x2[0]);
+                  else cfma(t[k], r[k], x2[0]);
+                  if (i + 1 < NORB) cfma(t[k], r[NORB + k], x2[1]);
                 }
+              }
+#pragma unroll
+              for (int k = 0; k < NORB; k++) {
+                acc[k].x += t[k].x;
+                acc[k].y += t[k].y;
               }
             }
           } else {
+            static_assert(NORB == 5, "10 orbitals: the branches above");
             if (cat) {
 #pragma unroll
               for (int i = 0; i < NORB; i++)
