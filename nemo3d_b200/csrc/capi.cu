@@ -101,6 +101,7 @@ static void free_ctx(Ctx *c) {
                   c->d_pen_scratch, c->d_fold_tmp};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (c->h_pinned) cudaFreeHost(c->h_pinned);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

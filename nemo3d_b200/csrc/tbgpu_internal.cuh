@@ -99,6 +99,9 @@ struct Ctx {
   unsigned int *d_counter = nullptr;
   int partial_cap = 0;
   int *d_status = nullptr;          // device error word
+  // pinned copies of alpha and beta during a solve (kept between solves)
+  double *h_pinned = nullptr;
+  size_t h_pinned_bytes = 0;
   // Lanczos state
   std::vector<double> alpha, beta;  // host copy of the last tridiagonal
   // stats
