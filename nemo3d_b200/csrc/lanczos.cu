@@ -28,6 +28,7 @@
 
 #include "host_par.h"
 #include "lanczos_step.cuh"
+#include "launch.cuh"
 #include "reduce.cuh"
 #include "tbgpu_internal.cuh"
 
@@ -109,13 +110,22 @@ __global__ void k_divide(long n2, const double2 *__restrict__ x, const double *d
   }
 }
 
+// k_update: what bounds it is bytes in flight (three vectors read, one
+// written; in L2 up to some 80k atoms, beyond that at 6.0 TB/s of HBM).  A
+// thread loads kUpdLoads 16-byte pieces of each vector before it computes,
+// kUpdBlocks blocks per SM: 17.0 -> 14.4 us at 45k atoms, 62.9 -> 55.3 at
+// 256k (one piece at a time, eight blocks; 4 x 4: 18.4 and 62.3, 2 x 6: 18.4
+// and 63.3, 6 x 2: 14.3 and 55.2 but 10.0 against 9.3 at 4k).
+constexpr int kUpdLoads = 3, kUpdBlocks = 4;
+
 // r_n = w - (alpha q + beta_prev q_prev), q = rc/bet[it], q_prev = rp/bet[it-1];
 // bet[it+1] = ||r_n||.  bet[0] is the norm of the start vector.
 template <typename VT>
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, kUpdBlocks)
     k_update(long n2, const VT *__restrict__ w, const VT *__restrict__ rc,
              const VT *__restrict__ rp, VT *__restrict__ rout,
              const double *alpha, double *bet, int it, double *partial, unsigned *counter) {
+  wait_for_previous();
   const double al = alpha[it], bprev = bet[it];
   const double iq = 1.0 / bprev;
   const double ip = it > 0 ? 1.0 / bet[it - 1] : 0.0;
@@ -130,27 +140,39 @@ __global__ void __launch_bounds__(kRedThreads)
   };
   const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const long nth = (long)gridDim.x * blockDim.x;
-  if constexpr (sizeof(VT) == sizeof(float2)) {
-    // complex floats two at a time: 16-byte loads and stores (the vectors
-    // start on 16-byte boundaries); each entry computes as one at a time
-    const long n4 = n2 / 2;
-    const float4 *w4 = reinterpret_cast<const float4 *>(w);
-    const float4 *c4 = reinterpret_cast<const float4 *>(rc);
-    const float4 *p4 = reinterpret_cast<const float4 *>(rp);
-    float4 *o4 = reinterpret_cast<float4 *>(rout);
-    for (long j = tid; j < n4; j += nth) {
-      const float4 a = w4[j], c = c4[j];
-      const float4 p = it > 0 ? p4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const VT r0 = entry(VT{a.x, a.y}, VT{c.x, c.y}, VT{p.x, p.y});
-      const VT r1 = entry(VT{a.z, a.w}, VT{c.z, c.w}, VT{p.z, p.w});
-      o4[j] = make_float4(r0.x, r0.y, r1.x, r1.y);
+  // 16 bytes at a time: a complex double, or two complex floats (the vectors
+  // start on 16-byte boundaries); each entry computes as one at a time
+  constexpr int E = 16 / int(sizeof(VT));
+  struct alignas(16) Piece { VT v[E]; };
+  const Piece *w4 = reinterpret_cast<const Piece *>(w), *c4 = reinterpret_cast<const Piece *>(rc);
+  const Piece *p4 = reinterpret_cast<const Piece *>(rp);
+  Piece *o4 = reinterpret_cast<Piece *>(rout);
+  const long n4 = n2 / E;
+  for (long j0 = tid; j0 < n4; j0 += kUpdLoads * nth) {
+    Piece a[kUpdLoads], c[kUpdLoads], q[kUpdLoads];
+#pragma unroll
+    for (int u = 0; u < kUpdLoads; u++) {
+      const long j = j0 + u * nth;
+      if (j < n4) {
+        a[u] = w4[j];
+        c[u] = c4[j];
+        if (it > 0) q[u] = p4[j];
+      }
     }
-    if ((n2 & 1) && tid == 0) {  // an odd length's last entry
-      const long j = n2 - 1;
-      rout[j] = entry(w[j], rc[j], it > 0 ? rp[j] : VT{});
+#pragma unroll
+    for (int u = 0; u < kUpdLoads; u++) {
+      const long j = j0 + u * nth;
+      if (j < n4) {
+        Piece o;
+#pragma unroll
+        for (int e = 0; e < E; e++) o.v[e] = entry(a[u].v[e], c[u].v[e], q[u].v[e]);
+        o4[j] = o;
+      }
     }
-  } else {
-    for (long j = tid; j < n2; j += nth) rout[j] = entry(w[j], rc[j], it > 0 ? rp[j] : VT{});
+  }
+  if (E > 1 && (n2 & 1) && tid == 0) {  // an odd length's last entry
+    const long j = n2 - 1;
+    rout[j] = entry(w[j], rc[j], it > 0 ? rp[j] : VT{});
   }
   grid_reduce<kRedThreads>(s, partial, counter, bet, it + 1, true);
 }
@@ -761,8 +783,9 @@ static int solve_t(Ctx &c, const SolveArgs &A, const double *r0_dev, double *val
       spmv_ev.push_back(e0);
       spmv_ev.push_back(e1);
     }
-    k_update<VT><<<rg, kRedThreads, 0, s>>>(n2, W, rc_, it > 0 ? rp_ : nullptr, ro, d_alpha, bet,
-                                            it, c.d_partial, c.d_counter);
+    launch_overlapped(k_update<VT>, std::min(rg, unsigned(c.sms * kUpdBlocks)), kRedThreads, 0, s,
+                      n2, W, rc_, it > 0 ? rp_ : nullptr, ro, d_alpha, bet, it, c.d_partial,
+                      c.d_counter);
     if (c.profiling) {
       cudaEvent_t e2 = nullptr;
       cudaEventCreate(&e2);
