@@ -95,7 +95,7 @@ static void free_ctx(Ctx *c) {
   if (!c) return;
   void *ptrs[] = {c->d_type, c->d_dsp, c->d_par, c->d_par_ok, c->d_site_index, c->d_atom_site,
                   c->d_nbr, c->d_site_m, c->d_surface, c->d_onsite, c->d_blocks, c->d_partial,
-                  c->d_counter, c->d_status, c->d_x, c->d_y, c->d_phase, c->d_wrap, c->d_bonds,
+                  c->d_counter, c->d_status, c->d_x, c->d_y, c->d_phase, c->d_wrap,
                   c->d_blocks32, c->d_onsite32, c->d_rc_order, c->d_start,
                   c->d_pen_blk, c->d_pen_ons, c->d_pen_ok,
                   c->d_pen_scratch, c->d_fold_tmp};

@@ -91,7 +91,7 @@ struct Ctx {
   float *d_blocks32 = nullptr;
   // H*x work order [natoms]: cations then anions, pencils visited in j-blocks,
   // and beside each atom its bonds (k_kind_order, topology.cu)
-  int *d_order = nullptr;           // (in d_bonds' allocation)
+  int *d_order = nullptr;           // (both in d_nbr's allocation)
   int4 *d_bonds = nullptr;
   long ncations = 0;
   // reduction scratch (per-block partials + completion counter)

@@ -222,9 +222,6 @@ static int build_work_order(Ctx &c, const int *first) {
   int *tmp = nullptr;  // at[2 npen + 1], cations[npen]
   TB_CUDA(cudaMallocAsync(&tmp, sizeof(int) * (3 * size_t(npen) + 1), c.stream));
   int *cations = tmp + 2 * size_t(npen) + 1;
-  // one allocation: the bonds, then the order
-  TB_CUDA(cudaMalloc(&c.d_bonds, (sizeof(int4) + sizeof(int)) * c.natoms));
-  c.d_order = reinterpret_cast<int *>(c.d_bonds + c.natoms);
   const unsigned wb = unsigned((npen + 7) / 8);
   k_kind_order<true><<<wb, 256, 0, c.stream>>>(npen, per, first, c.d_site_m, c.d_nbr, nullptr,
                                                cations, nullptr, nullptr);
@@ -269,7 +266,10 @@ int build_topology(Ctx &c) {
   if (rc == TBGPU_OK) {
     TB_CUDA(cudaMalloc(&c.d_site_index, sizeof(int) * ns));
     TB_CUDA(cudaMalloc(&c.d_atom_site, sizeof(int) * natoms));
-    TB_CUDA(cudaMalloc(&c.d_nbr, sizeof(int4) * natoms));
+    // one allocation: neighbours, bonds and work order
+    TB_CUDA(cudaMalloc(&c.d_nbr, (2 * sizeof(int4) + sizeof(int)) * natoms));
+    c.d_bonds = c.d_nbr + natoms;
+    c.d_order = reinterpret_cast<int *>(c.d_bonds + natoms);
     TB_CUDA(cudaMalloc(&c.d_site_m, natoms));
     TB_CUDA(cudaMalloc(&c.d_surface, natoms));
     k_finalize<<<blocks, threads, 0, c.stream>>>(g, ns, flag, index, c.d_site_index,
