@@ -63,10 +63,9 @@ METRIC = "s to 8 band-edge eigenpairs at <=1e-6 eV vs plain FP64 GPU Lanczos; Sp
 # x read once, y written once): FP64 1864 + 640, complex-float 936 + 320.
 BYTES_PER_ATOM = {64: 2504, 32: 1256}
 # DRAM bytes per atom of one H*x launch, measured with ncu (dram__bytes_read
-# + dram__bytes_write, one launch, cold L2) on the 384,000-atom profile case
-# and scaled by atoms: the float lane kernel 488.6 MB, the FP64 default
-# kernel 3054 B/atom at full size.
-NCU_TRAFFIC_PER_ATOM = {32: 1272, 64: 3054}
+# + dram__bytes_write, one launch, cold L2) and scaled by atoms: the ring
+# kernel at 1.99M atoms (float) and at 1.02M (FP64).
+NCU_TRAFFIC_PER_ATOM = {32: 1377, 64: 2610}
 # one complex vector per atom (20 entries: FP64 320 B, complex float 160 B) and
 # the stored blocks + on-site records + neighbour columns per atom (B_H)
 VEC_PER_ATOM = {64: 320, 32: 160}
@@ -81,8 +80,8 @@ NVEC = 8
 # the 1.02M-atom dome: 8 hole and 8 electron states
 SOLVE_8X8 = dict(SOLVE, requested1=8, requested2=8, emin1=0.95, emax1=1.06, emin2=1.44,
                  emax2=1.56, imax=30000)
-# the mixed-precision solver: float store and vectors, H*x variant 5 (lane
-# per atom and spin), eigenvector pass 1 (regeneration, 4 columns,
+# the mixed-precision solver: float store and vectors, H*x variant 5 (the
+# ring kernel), eigenvector pass 1 (regeneration, 4 columns,
 # 256-iteration segments)
 MIXED_VARIANT = 5
 MIXED_VEC_PASS = (1, 4, 256)
@@ -501,7 +500,7 @@ def run_ours(args, rank, world, local_rank):
                          "peak_source": pk_kind,
                          "traffic": NCU_TRAFFIC_PER_ATOM[bits] * natoms,
                          "kernel": "H*x with fused alpha (first pass), "
-                                   + ("complex-float lane kernel" if mixed else "FP64"),
+                                   + ("complex-float ring kernel" if mixed else "FP64"),
                          "algorithmic_bytes": BYTES_PER_ATOM[bits] * natoms,
                          "avg_launch_ms": spmv_ms},
             "clocks": clk.summary(),
@@ -590,7 +589,7 @@ def _event_time(fn, reps, stream_ctx):
 
 def run_extra(args):
     """Measurements beside the headline (one JSON line each), on one GPU:
-    kernels   H*x of the 1.02M-atom dome: FP64 store (warp-staged and two-cell unit
+    kernels   H*x of the 1.02M-atom dome: FP64 store (ring, lane-gather and pencil
               kernels), float store with float
               vectors, recompute in FP64 and in float
     mixed2M   the same dome at 72 x 72 x 48 cells (1,990,656 atoms): plain FP64
@@ -659,19 +658,14 @@ def run_extra(args):
         f32o = dict(ham_bits=32, lanczos_bits=32)
         for name, opts, f32, var, st in (
                 ("fp64 store", {}, False, 0, st1),
-                ("fp64 store, two-cell units (variant 3)", {}, False, 3, st1),
-                ("fp64 store, every piece by cp.async (variant 4)", {}, False, 4, st1),
-                ("fp64 store, lane per atom and spin (variant 5)", {}, False, 5, st1),
+                ("fp64 store, lane gather (variant 1)", {}, False, 1, st1),
                 ("fp64 store, pencil layout (variant 6)", {}, False, 6, st1),
                 ("float store, float vectors", dict(ham_bits=32, lanczos_bits=32), True, 0, st1),
-                ("float store, float vectors, lane per atom and spin (variant 5)",
-                 dict(ham_bits=32, lanczos_bits=32), True, 5, st1),
                 ("float store, float vectors, pencil layout (variant 6)",
                  dict(ham_bits=32, lanczos_bits=32), True, 6, st1),
                 ("recompute fp64", dict(recompute=True), False, 0, st1),
                 ("recompute float", dict(recompute=True, lanczos_bits=32), True, 0, st1),
-                ("2M dot, float store, float vectors, lane per atom and spin (variant 5)",
-                 f32o, True, 5, st2),
+                ("2M dot, float store, float vectors", f32o, True, 0, st2),
                 ("2M dot, float store, float vectors, pencil layout (variant 6)", f32o, True, 6,
                  st2),
                 ("2M dot, float store, float vectors, pencil layout, staged rows (variant 7)",
@@ -711,12 +705,12 @@ def run_extra(args):
         f32 = dict(ham_bits=32, lanczos_bits=32)
         # (name, options, H*x variant, eigenvector pass (mode, columns,
         # segment) or None, tolerance)
-        variants = [("fp64 (warp-staged kernel, second run for the vectors)", {}, 0, None, 1e-7),
+        variants = [("fp64 (ring kernel, second run for the vectors)", {}, 0, None, 1e-7),
                     ("fp64, pencil kernel", {}, 6, None, 1e-7),
                     ("fp64, pencil kernel, regenerated vectors P=2 L=256", {}, 6, (1, 2, 256),
                      1e-7),
-                    ("mixed, float store, warp-staged kernel", f32, 0, None, 1e-7),
-                    ("mixed, float store, lane kernel, regenerated vectors P=4 L=256", f32, 5,
+                    ("mixed, float store, second run for the vectors", f32, 0, None, 1e-7),
+                    ("mixed, float store, ring kernel, regenerated vectors P=4 L=256", f32, 5,
                      (1, 4, 256), 1e-7),
                     ("mixed, float store, pencil kernel, regenerated vectors P=4 L=256", f32, 6,
                      (1, 4, 256), 1e-7),
