@@ -38,7 +38,7 @@
 // passes); lane per (atom, spin) with rows straight from global memory, one
 // tag lookup per lane and load (float, 381k atoms: 0.181 against 0.118 ms);
 // lane-gather, 5-orbital dots, 0.43M atoms: 0.200 against 0.104 ms; a staged
-// block product of 8 vectors, 66k atoms: 0.296 against 0.183 ms.
+// block product of 8 vectors, 66k atoms: 0.296 against 0.177 ms.
 //
 // Every column of a launch computes as a one-vector launch would, operation
 // for operation, so regenerated recurrences are bit-identical to the first
@@ -786,19 +786,21 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         } else {
           __syncwarp();
-        for_lines<APW * P, S::XPC>(
-            ag, [&](int s, int) { return __shfl_sync(0xffffffffu, valid ? la : -1, (s / P) * LPA); },
-            [&](int a, int s, int pc) {
-              const uintptr_t dst = reinterpret_cast<uintptr_t>(A.y[P == 1 ? 0 : s % P]) + long(max(a, 0)) * S::XB;
-              line_chunk<S::XCH, S::XCH_B, S::XMASK>(dst, sub, pc, [&](int o) {
-                const unsigned char *src = own_p + s * S::XP + o + (S::SP > S::SEG && o >= S::SEG ? S::SP - S::SEG : 0);
-                if (a < 0) return;
-                if constexpr (S::XCH_B == 16)
-                  *reinterpret_cast<float4 *>(dst + o) = *reinterpret_cast<const float4 *>(src);
-                else
-                  *reinterpret_cast<float2 *>(dst + o) = *reinterpret_cast<const float2 *>(src);
+          for_lines<APW * P, S::XPC>(
+              ag, [&](int s, int) { return __shfl_sync(0xffffffffu, valid ? la : -1, (s / P) * LPA); },
+              [&](int a, int s, int pc) {
+                const uintptr_t dst =
+                    reinterpret_cast<uintptr_t>(A.y[P == 1 ? 0 : s % P]) + long(max(a, 0)) * S::XB;
+                line_chunk<S::XCH, S::XCH_B, S::XMASK>(dst, sub, pc, [&](int o) {
+                  const unsigned char *src =
+                      own_p + s * S::XP + o + (S::SP > S::SEG && o >= S::SEG ? S::SP - S::SEG : 0);
+                  if (a < 0) return;
+                  if constexpr (S::XCH_B == 16)
+                    *reinterpret_cast<float4 *>(dst + o) = *reinterpret_cast<const float4 *>(src);
+                  else
+                    *reinterpret_cast<float2 *>(dst + o) = *reinterpret_cast<const float2 *>(src);
+                });
               });
-            });
         }
         // (the own slot is free once bond 0 of the next task is arrived on)
       }

@@ -166,3 +166,38 @@ def test_order_of_overlapped_launches(name, captured):
     torch.cuda.synchronize()
     for got, w in zip(bufs, want):
         assert torch.equal(got, w)
+
+
+@pytest.mark.parametrize("name", ["1x1x1", "5x3x7_vacancies", "17x9x11"])
+@pytest.mark.parametrize("model", ["sp3d5s*_so", "sp3s*"])
+@pytest.mark.parametrize("bits", [64, 32])
+def test_recurrence_matches_oracle(name, model, bits):
+    """alpha and beta of six Lanczos steps (product, update, overlapped
+    launches; vectors of odd and even lengths, fewer entries than threads)
+    against the same steps on the oracle's product.  Each step adds at most
+    one product's error (the bars above) to the vector, and the vector of the
+    step before enters once more, so seven bars a step are allowed."""
+    import torch
+    its = 6
+    opts = dict(ham_bits=32, lanczos_bits=32) if bits == 32 else {}
+    g, o, scale = _pair(name, model, **opts)
+    rng = np.random.default_rng(9)
+    r = rng.uniform(-1, 1, 2 * g.n)
+    r0 = torch.from_numpy(r.copy()).cuda()
+    g.eigensolve_lanczos_dev(r0.data_ptr(), imax=its + 1, emin1=1.0, emax1=1.1, emin2=1.4,
+                             emax2=1.5)
+    alpha, beta = g.tridiagonal(its + 1)
+    r /= np.linalg.norm(r)
+    prev, bprev, a_ref, b_ref = np.zeros_like(r), 0.0, [], []
+    for _ in range(its):
+        w = o.hx(r, 0.0)
+        a = float(w @ r)
+        w = w - a * r - bprev * prev
+        b = float(np.linalg.norm(w))
+        prev, bprev, r = r, b, w / b
+        a_ref.append(a)
+        b_ref.append(b)
+    bar = 45e-12 * scale if bits == 64 else 48 * 2.0 ** -24 * 45 * scale
+    assert len(alpha) == its
+    assert np.abs(alpha - a_ref).max() <= 7 * its * bar
+    assert np.abs(beta[:its] - b_ref).max() <= 7 * its * bar
