@@ -1,0 +1,59 @@
+"""Products whose time must not exceed that of a product that does more.
+
+A time of one shape is compared with the time of another on the same GPU in
+the same process, so the bars hold on any clock: a block of p vectors takes no
+longer than a block of 8 on the same structure (1.35 times allowed; measured
+0.75 to 1.13, and 1.6 to 2.4 with the staging that took line after line of a
+flat count for p = 3, 5, 6 and 7).
+"""
+import numpy as np
+import pytest
+
+from nemo3d_b200 import materials, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _ham(cells, model, **opts):
+    """An InGaAs alloy cube of `cells`^3 conventional cells, on torch's stream."""
+    import torch
+    from nemo3d_b200.tbgpu import Hamiltonian
+    fam = "sps" if model.startswith("sp3s*") else "spds"
+    rng = np.random.default_rng(3)
+    t = np.empty((cells,) * 3 + (8,), np.uint8)
+    t[..., :4] = np.where(rng.random((cells,) * 3 + (4,)) < 0.5, materials.SPECIES["In"],
+                          materials.SPECIES["Ga"])
+    t[..., 4:] = materials.SPECIES["As"]
+    st = workloads.Structure(cells, cells, cells, (workloads.A_GAAS,) * 3, (False,) * 3, t,
+                             rng.normal(0, 0.004, t.shape + (3,)))
+    g = Hamiltonian(st, model, [materials.MATERIALS["GaAs_" + fam],
+                                materials.MATERIALS["InAs_" + fam]], **opts)
+    g.set_stream(torch.cuda.current_stream().cuda_stream)
+    return g
+
+
+def _time(fn, calls=200, rounds=7):
+    """us per call: the shortest of a few rounds of calls in a row."""
+    import torch
+    a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    best = float("inf")
+    for _ in range(rounds):
+        a.record()
+        for _ in range(calls):
+            fn()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3 / calls)
+    return best
+
+
+@pytest.mark.parametrize("model", ["sp3d5s*_so", "sp3d5s*"])
+def test_narrow_blocks_take_no_longer_than_wide_ones(model):
+    import torch
+    g = _ham(6, model)
+    x = torch.rand(8 * 2 * g.n, dtype=torch.float64, device="cuda")
+    y = torch.empty_like(x)
+    t = {p: _time(lambda: g.hx_block_dev(p, x.data_ptr(), y.data_ptr(), 0.3))
+         for p in range(2, 9)}
+    print(model, {p: round(v, 2) for p, v in t.items()})
+    assert max(t.values()) <= 1.35 * t[8], t
