@@ -7,8 +7,9 @@
 // product matmat_mult (nemo3d/src/base/h_cmat_mult.c:21).
 //
 //  * A task is 32 / (vectors * spins * H) atoms of one kind (all cations or
-//    all anions), one lane per atom, vector and spin (H = 2 lanes for single
-//    double vectors of the 10-orbital models, see ring_split).  A cation
+//    all anions; 8 or 16 for 32 on small structures, see run_one), one lane per atom,
+//    vector and spin (H = 2 lanes for single double vectors of the 10-orbital
+//    models, see ring_split).  A cation
 //    lane streams the rows of its block against its neighbour's x segment; an
 //    anion lane streams the rows of the block its cation neighbour stores and
 //    scales each by that neighbour's x entry (the transposed product).  A lane
@@ -111,14 +112,14 @@ __host__ __device__ constexpr int ring_split(int norb, int p, int vector_bytes) 
   return norb == 10 && p == 1 && vector_bytes == 16 ? 2 : 1;
 }
 
-// Shared-memory geometry of a configuration (bytes)
-template <int NORB, int NSPIN, int P, typename HT, typename VT, bool UPD>
+// Shared-memory geometry of a configuration (bytes), tasks of TA atoms at most
+template <int NORB, int NSPIN, int P, typename HT, typename VT, bool UPD, int TA>
 struct RingShape {
   static constexpr int NB = NORB * NSPIN;
   static constexpr int H = ring_split(NORB, P, int(sizeof(VT)));
   static constexpr int NO = NORB / H;                 // orbitals per lane
   static constexpr int LPA = P * NSPIN * H;           // lanes per atom
-  static constexpr int APW = 32 / LPA;                // atoms per task
+  static constexpr int APW = 32 / LPA < TA ? 32 / LPA : TA;  // atoms per task
   static constexpr int BLKB = NORB * NORB * int(sizeof(HT));
   // a block's 16-byte chunks (a block of the 5-orbital models may start
   // inside one), and their odd pitch
@@ -266,7 +267,7 @@ struct TaskMeta {
 };
 
 template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool UPD, bool PHASE,
-          int PAIRS, int SLOTS>
+          int TA, int PAIRS, int SLOTS>
 __global__ void __launch_bounds__(PAIRS * 64, 1)
     k_hx_ring(int ncat, int nan, const int *__restrict__ order, const int4 *__restrict__ bonds,
               const HT *__restrict__ onsite, const HT *__restrict__ blocks,
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
               unsigned int *counter, double *alpha_out, int alpha_idx,
               const double2 *__restrict__ phase, const unsigned char *__restrict__ wrap,
               const unsigned char *__restrict__ skip, int *status) {
-  using S = RingShape<NORB, NSPIN, P, HT, VT, UPD>;
+  using S = RingShape<NORB, NSPIN, P, HT, VT, UPD, TA>;
   using RT = typename RealOf<VT>::T;
   constexpr int NB = S::NB, APW = S::APW, LPA = S::LPA, H = S::H, NO = S::NO;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -842,13 +843,14 @@ struct RingLaunch {
   int aidx;
 };
 
-template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool UPD, bool PHASE>
+template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool UPD, bool PHASE,
+          int TA = 32>
 int run_ring(Ctx &c, const RingCols<VT, P> &A, RingLaunch L, cudaStream_t s) {
-  using S = RingShape<NORB, NSPIN, P, HT, VT, UPD>;
+  using S = RingShape<NORB, NSPIN, P, HT, VT, UPD, TA>;
   constexpr int SLOTS = kSlots, PAIRS = ring_pairs<S>(NORB == 10 && sizeof(VT) == 16);
   constexpr int smem = PAIRS * S::pair_bytes(SLOTS);
   static_assert(PAIRS >= 1, "a task does not fit shared memory");
-  const auto kernel = k_hx_ring<NORB, NSPIN, P, HT, VT, DOT, UPD, PHASE, PAIRS, SLOTS>;
+  const auto kernel = k_hx_ring<NORB, NSPIN, P, HT, VT, DOT, UPD, PHASE, TA, PAIRS, SLOTS>;
   static std::atomic<unsigned long long> attr_done{0};
   if (ensure_smem_attr(attr_done, c.device, kernel, smem)) return TBGPU_E_CUDA;
   const int ncat = int(c.ncations), nan = int(c.natoms - c.ncations);
@@ -869,19 +871,45 @@ int run_ring(Ctx &c, const RingCols<VT, P> &A, RingLaunch L, cudaStream_t s) {
   return TBGPU_OK;
 }
 
-template <int NORB, int NSPIN, typename HT, typename VT>
-int run_one(Ctx &c, const VT *x, VT *y, int it, const RingLaunch &L, cudaStream_t s) {
+template <int NORB, int NSPIN, typename HT, typename VT, int TA>
+int run_tasks(Ctx &c, const VT *x, VT *y, int it, const RingLaunch &L, cudaStream_t s) {
   RingCols<VT, 1> A{};
   A.x[0] = x;
   A.y[0] = y;
   A.it[0] = it;
   if constexpr (sizeof(VT) == sizeof(double2)) {
     if (c.bloch)
-      return L.alpha_out ? run_ring<NORB, NSPIN, 1, HT, VT, true, false, true>(c, A, L, s)
-                         : run_ring<NORB, NSPIN, 1, HT, VT, false, false, true>(c, A, L, s);
+      return L.alpha_out ? run_ring<NORB, NSPIN, 1, HT, VT, true, false, true, TA>(c, A, L, s)
+                         : run_ring<NORB, NSPIN, 1, HT, VT, false, false, true, TA>(c, A, L, s);
   }
-  return L.alpha_out ? run_ring<NORB, NSPIN, 1, HT, VT, true, false, false>(c, A, L, s)
-                     : run_ring<NORB, NSPIN, 1, HT, VT, false, false, false>(c, A, L, s);
+  return L.alpha_out ? run_ring<NORB, NSPIN, 1, HT, VT, true, false, false, TA>(c, A, L, s)
+                     : run_ring<NORB, NSPIN, 1, HT, VT, false, false, false, TA>(c, A, L, s);
+}
+
+// One vector.  A product with fewer tasks than warp pairs takes as long as one
+// task, whose producer copies for every atom the task has room for: 8 or 16
+// with several lanes an atom, 32 with one (5 orbitals or float vectors, no
+// spin).  Those 32 make way for tasks of
+//  * 8 atoms while the SMs get at most four of them (216 atoms, sp3s*: 4.9 us,
+//    5.7 with 16, 7.4 with 32; float sp3d5s* 5.4, 6.3 and 7.2.  At 5,832 and
+//    8,000 atoms float sp3d5s* is at 6.0 to 6.4 with either, so the line is
+//    where each scheduler has one pair),
+//  * 16 atoms while the warp pairs get at most one (the 10-orbital models:
+//    eight a SM).  17,576 atoms, sp3s*: 6.7 us, 7.9 with 32; float sp3d5s* 7.6
+//    against 8.1.  Past the line the second round costs more than it saves:
+//    32,768 atoms, sp3s*, 10.7 against 8.8; float sp3d5s*, 27,000, 9.2 against
+//    8.8.
+// Results are the same bit for bit, only the fused dot sums in another order.
+template <int NORB, int NSPIN, typename HT, typename VT>
+int run_one(Ctx &c, const VT *x, VT *y, int it, const RingLaunch &L, cudaStream_t s) {
+  if constexpr (RingShape<NORB, NSPIN, 1, HT, VT, false, 32>::APW == 32) {
+    const int kind = int(std::max(c.ncations, c.natoms - c.ncations));
+    auto per_sm = [&](int atoms, int tasks) { return 2 * cdiv(kind, atoms) <= tasks * c.sms; };
+    if (per_sm(8, 4)) return run_tasks<NORB, NSPIN, HT, VT, 8>(c, x, y, it, L, s);
+    if (per_sm(16, NORB == 5 ? 12 : 8))
+      return run_tasks<NORB, NSPIN, HT, VT, 16>(c, x, y, it, L, s);
+  }
+  return run_tasks<NORB, NSPIN, HT, VT, 32>(c, x, y, it, L, s);
 }
 
 template <typename HT, typename VT>
