@@ -75,3 +75,69 @@ def test_spinless_product_takes_no_longer_than_the_spin_model(store, single):
         t[model] = _time(lambda: call(x.data_ptr(), y.data_ptr(), 0.3))
     print(store, single, {m: round(v, 2) for m, v in t.items()})
     assert t["sp3s*"] <= 1.12 * t["sp3s*_so"], t
+
+
+@pytest.mark.parametrize("model", list(materials.BAND_MODELS))
+def test_product_with_dot_takes_less_than_two_products(model):
+    """216 atoms: the allocation-free product with its dot (one reduction more
+    than the product) against 1.8 products; measured 1.46 to 1.57, and 2.0 to
+    2.5 with the counter cleared by a memset."""
+    import ctypes as C
+    import torch
+    from nemo3d_b200 import tbgpu
+    f = tbgpu._lib().tbgpu_hx_dot_noalloc
+    f.argtypes = [C.c_void_p, C.c_double, C.c_void_p, C.c_void_p, C.c_void_p]
+    f.restype = C.c_int
+    g = _ham(3, model)
+    x = torch.rand(2 * g.n, dtype=torch.float64, device="cuda")
+    y, dot = torch.empty_like(x), torch.zeros(1, dtype=torch.float64, device="cuda")
+    one = _time(lambda: g.hx_dev(x.data_ptr(), y.data_ptr(), 0.3))
+    both = _time(lambda: f(g._ctx, 0.3, x.data_ptr(), y.data_ptr(), dot.data_ptr()))
+    print(model, round(one, 2), round(both, 2))
+    assert both <= 1.8 * one, (one, both)
+
+
+@pytest.mark.parametrize("cells", [1, 6])
+def test_product_with_dot_in_a_row_and_captured(cells):
+    """Calls in a row, each on the result of the one before, and the same calls
+    replayed from a graph: dots and vectors as with a synchronisation after
+    every call."""
+    import ctypes as C
+    import torch
+    from nemo3d_b200 import tbgpu
+    f = tbgpu._lib().tbgpu_hx_dot_noalloc
+    f.argtypes = [C.c_void_p, C.c_double, C.c_void_p, C.c_void_p, C.c_void_p]
+    f.restype = C.c_int
+    g = _ham(cells, "sp3d5s*_so")
+    x = torch.from_numpy(np.random.default_rng(4).uniform(-1, 1, 2 * g.n)).cuda()
+    a, b = x.clone(), torch.zeros_like(x)
+    dots = torch.zeros(8, dtype=torch.float64, device="cuda")
+
+    def work(sync):
+        a.copy_(x)
+        for k in range(8):
+            src, dst = (a, b) if k % 2 == 0 else (b, a)
+            assert f(g._ctx, 0.1 * k, src.data_ptr(), dst.data_ptr(),
+                     dots.data_ptr() + 8 * k) == 0
+            if sync:
+                torch.cuda.synchronize()
+
+    work(True)
+    want = [t.clone() for t in (a, b, dots)]
+    assert dots.abs().min() > 0
+    run = torch.cuda.Stream()
+    run.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(run):
+        g.set_stream(run.cuda_stream)
+        dots.zero_()
+        work(False)
+        torch.cuda.synchronize()
+        assert all(torch.equal(t, w) for t, w in zip((a, b, dots), want))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=run):
+            work(False)
+        dots.zero_()
+        graph.replay()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(t, w) for t, w in zip((a, b, dots), want))
