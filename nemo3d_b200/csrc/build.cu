@@ -214,8 +214,8 @@ __global__ void k_to_float(long n, const double *__restrict__ in, float *__restr
     out[i] = float(in[i]);
 }
 
-static int to_float(Ctx &c, long n, const double *in, float **out) {
-  TB_CUDA(cudaMalloc(out, sizeof(float) * n));
+static int to_float(Ctx &c, long n, const double *in, float **out, size_t room = 0) {
+  TB_CUDA(cudaMalloc(out, sizeof(float) * n + room));
   k_to_float<<<1184, 256, 0, c.stream>>>(n, in, *out);
   TB_CUDA(cudaGetLastError());
   return TBGPU_OK;
@@ -229,8 +229,12 @@ int assemble(Ctx &c) {
   if (c.lanczos_f32 && !c.recompute && !c.ham_fp32) return set_error(TBGPU_E_UNSUPPORTED);
   // recompute: the blocks are not stored; the assembly still runs the bond
   // kernel for the on-site strain corrections
-  if (!c.recompute)
-    TB_CUDA(cudaMalloc(&c.d_blocks, sizeof(double) * na * 4 * c.norb * c.norb));
+  const long nblk = na * 4 * c.norb * c.norb;
+  const size_t room = kOrderBytes * na;  // the work order, behind the blocks that stay
+  if (!c.recompute) {
+    if (na >= (1L << 29)) return set_error(TBGPU_E_UNSUPPORTED);  // block numbers are ints
+    TB_CUDA(cudaMalloc(&c.d_blocks, sizeof(double) * nblk + (c.ham_fp32 ? 0 : room)));
+  }
   TB_CUDA(cudaMalloc(&c.d_onsite, sizeof(double) * na * c.ons));
   int rc = TBGPU_E_UNSUPPORTED;
   if (c.norb == 10 && c.nspin == 2) rc = assemble_t<10, 2>(c);
@@ -239,8 +243,10 @@ int assemble(Ctx &c) {
   else if (c.norb == 5 && c.nspin == 1) rc = assemble_t<5, 1>(c);
   else return set_error(rc);
   if (!rc && (c.recompute || c.lanczos_f32)) rc = build_recompute_order(c);
-  if (rc || !c.ham_fp32) return rc;
-  if ((rc = to_float(c, na * 4 * c.norb * c.norb, c.d_blocks, &c.d_blocks32))) return rc;
+  if (rc || c.recompute) return rc;
+  if (!c.ham_fp32) return build_work_order(c, c.d_blocks + nblk, c.d_status + 1);
+  if ((rc = to_float(c, nblk, c.d_blocks, &c.d_blocks32, room))) return rc;
+  if ((rc = build_work_order(c, c.d_blocks32 + nblk, c.d_status + 1))) return rc;
   if ((rc = to_float(c, na * c.ons, c.d_onsite, &c.d_onsite32))) return rc;
   TB_CUDA(cudaStreamSynchronize(c.stream));
   cudaFree(c.d_blocks);

@@ -151,7 +151,7 @@ static int create(const tbgpu_geom *g, const tbgpu_model *m, bool dev, tbgpu_ctx
   if (cudaMalloc(&c->d_par, npar * kNPAR * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->d_par_ok, npar) != cudaSuccess ||
       cudaMalloc(&c->d_counter, sizeof(unsigned)) != cudaSuccess ||
-      cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess)
+      cudaMalloc(&c->d_status, 2 * sizeof(int)) != cudaSuccess)
     return fail(TBGPU_E_NOMEM);
   if (!dev) {  // species ids index the parameter table
     for (size_t i = 0; i < ns; i++)
@@ -165,7 +165,7 @@ static int create(const tbgpu_geom *g, const tbgpu_model *m, bool dev, tbgpu_ctx
           cudaSuccess ||
       cudaMemcpy(c->d_par_ok, m->par_ok, npar, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(c->d_counter, 0, sizeof(unsigned)) != cudaSuccess ||
-      cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess)
+      cudaMemset(c->d_status, 0, 2 * sizeof(int)) != cudaSuccess)
     return fail(TBGPU_E_CUDA);
   *out = reinterpret_cast<tbgpu_ctx *>(c);
   return TBGPU_OK;
@@ -223,10 +223,11 @@ int tbgpu_build_hamiltonian(tbgpu_ctx *ctx) {
   if (rc == TBGPU_OK) rc = ensure_partials(c, int(c.natoms / 8 + 65536));
   cudaEventRecord(e1, c.stream);
   if (cudaStreamSynchronize(c.stream) != cudaSuccess && rc == TBGPU_OK) rc = set_error(TBGPU_E_CUDA);
-  int st = 0;
-  if (rc == TBGPU_OK && cudaMemcpy(&st, c.d_status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+  int st[2] = {0, 0};  // status, cations
+  if (rc == TBGPU_OK && cudaMemcpy(st, c.d_status, sizeof(st), cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = set_error(TBGPU_E_CUDA);
-  if (rc == TBGPU_OK && st != 0) rc = set_error(st);
+  if (rc == TBGPU_OK && st[0] != 0) rc = set_error(st[0]);
+  c.ncations = st[1];
   float ms = 0.f;
   cudaEventElapsedTime(&ms, e0, e1);
   c.stats.build_ms = ms;

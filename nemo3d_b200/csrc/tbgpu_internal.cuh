@@ -91,14 +91,14 @@ struct Ctx {
   float *d_blocks32 = nullptr;
   // H*x work order [natoms]: cations then anions, pencils visited in j-blocks,
   // and beside each atom its bonds (k_kind_order, topology.cu)
-  int *d_order = nullptr;           // (both in d_nbr's allocation)
+  int *d_order = nullptr;           // (both behind the stored blocks)
   int4 *d_bonds = nullptr;
   long ncations = 0;
   // reduction scratch (per-block partials + completion counter)
   double *d_partial = nullptr;
   unsigned int *d_counter = nullptr;
   int partial_cap = 0;
-  int *d_status = nullptr;          // device error word
+  int *d_status = nullptr;          // device error word, count of cations
   // pinned copies of alpha and beta during a solve (kept between solves)
   double *h_pinned = nullptr;
   size_t h_pinned_bytes = 0;
@@ -209,6 +209,8 @@ int band_eigenvalues(int n, int kd, const std::complex<double> *ab, double vl, d
 
 // topology.cu
 int build_topology(Ctx &c);
+constexpr size_t kOrderBytes = sizeof(int4) + sizeof(int);  // of the work order, an atom
+int build_work_order(Ctx &c, void *room, int *ncations);
 int build_phases(Ctx &c);  // fills d_phase for c.kvec
 // build.cu
 int assemble(Ctx &c);

@@ -142,24 +142,38 @@ constexpr int kPencilBlock = 8;
 // each kind in the pencil order above; beside each atom its bonds, four times
 // the neighbour for a cation, the block its neighbour stores the bond in
 // (neighbour * 4 + slot) for an anion, -1 for none.  Built on the device in
-// three launches (the order was built on the host and copied before, two
-// round trips).  first[p * per] is the first atom of pencil p, per sites each
-// (first[npen * per] = natoms).
+// three launches without a wait: the host reads the count of cations where it
+// reads the build's status.  Only a stored Hamiltonian has the order, behind
+// its blocks: 20 bytes an atom in an allocation of their own are a further
+// mapping of device memory (building 65,688 atoms: 3.1 against 2.75 ms).
 
-// cations[p] (COUNT), or the pencil's entries from at[0][p] and at[1][p] (plus
-// the number of cations); one warp per pencil
+// first atom on a site not below s (atoms are numbered in site order)
+__device__ __forceinline__ int first_atom(int natoms, const int *__restrict__ atom_site, long s) {
+  int lo = 0, hi = natoms;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(atom_site + mid) < s) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// cations[p] and anions[p] (COUNT), or the pencil's entries from at[0][p] and
+// at[1][p] (plus the number of cations); one warp per pencil, per sites each
 template <bool COUNT>
-__global__ void k_kind_order(int npen, long per, const int *__restrict__ first,
+__global__ void k_kind_order(int natoms, int npen, long per, const int *__restrict__ atom_site,
                              const unsigned char *__restrict__ site_m,
                              const int4 *__restrict__ nbr, const int *__restrict__ at,
-                             int *__restrict__ cations, int *__restrict__ order,
+                             const int *__restrict__ ncations, int *__restrict__ cations,
+                             int *__restrict__ anions, int *__restrict__ order,
                              int4 *__restrict__ bonds) {
   const int p = int(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   if (p >= npen) return;
   const int lane = threadIdx.x & 31;
   const unsigned before = (1u << lane) - 1u;
-  const int start = first[p * per], end = first[(p + 1) * per];
-  int nc = COUNT ? 0 : at[p], na = COUNT ? 0 : at[npen + p] + at[2 * npen];
+  const int start = first_atom(natoms, atom_site, p * per);
+  const int end = first_atom(natoms, atom_site, (p + 1) * per);
+  int nc = COUNT ? 0 : at[p], na = COUNT ? 0 : at[npen + p] + *ncations;
   for (int a0 = start; a0 < end; a0 += 32) {
     const int a = a0 + lane;
     const bool in = a < end;
@@ -176,15 +190,18 @@ __global__ void k_kind_order(int npen, long per, const int *__restrict__ first,
     nc += __popc(cat);
     na += __popc(an);
   }
-  if (COUNT && lane == 0) cations[p] = nc;
+  if (COUNT && lane == 0) {
+    cations[p] = nc;
+    anions[p] = na;
+  }
 }
 
 // at[0][p], at[1][p]: cations and anions of the pencils visited before p;
-// at[2 npen]: all cations.  One block.
+// ncations: all of them.  One block.
 constexpr int kScanThreads = 1024;
 __global__ void __launch_bounds__(kScanThreads)
-    k_kind_scan(int nx, int ny, long per, const int *__restrict__ first,
-                const int *__restrict__ cations, int *__restrict__ at) {
+    k_kind_scan(int nx, int ny, const int *__restrict__ cations, const int *__restrict__ anions,
+                int *__restrict__ at, int *__restrict__ ncations) {
   using Scan = cub::BlockScan<int, kScanThreads>;
   __shared__ typename Scan::TempStorage tmp;
   const int npen = nx * ny, full = ny / kPencilBlock * kPencilBlock;
@@ -198,7 +215,7 @@ __global__ void __launch_bounds__(kScanThreads)
       const int jb = whole ? v / (w * nx) * kPencilBlock : full;
       p = r / w * ny + jb + r % w;
       cat = cations[p];
-      an = first[(p + 1) * per] - first[p * per] - cat;
+      an = anions[p];
     }
     int c0, a0, ct, t;
     Scan(tmp).ExclusiveSum(cat, c0, ct);
@@ -212,29 +229,29 @@ __global__ void __launch_bounds__(kScanThreads)
     nc += ct;
     na += t;
   }
-  if (threadIdx.x == 0) at[2 * npen] = nc;
+  if (threadIdx.x == 0) *ncations = nc;
 }
 
-static int build_work_order(Ctx &c, const int *first) {
-  if (c.natoms >= (1L << 29)) return set_error(TBGPU_E_UNSUPPORTED);  // block ids are ints
-  const int npen = c.nx * c.ny;
+// into room (natoms * kOrderBytes, 16-byte aligned) behind the stored blocks;
+// *ncations (device) receives the count of cations
+int build_work_order(Ctx &c, void *room, int *ncations) {
+  const int na = int(c.natoms), npen = c.nx * c.ny;
   const long per = long(c.nz) * 8;
-  int *tmp = nullptr;  // at[2 npen + 1], cations[npen]
-  TB_CUDA(cudaMallocAsync(&tmp, sizeof(int) * (3 * size_t(npen) + 1), c.stream));
-  int *cations = tmp + 2 * size_t(npen) + 1;
+  c.d_bonds = static_cast<int4 *>(room);
+  c.d_order = reinterpret_cast<int *>(c.d_bonds + na);
+  int *tmp = nullptr;  // at[2 npen], cations[npen], anions[npen]
+  TB_CUDA(cudaMallocAsync(&tmp, sizeof(int) * 4 * size_t(npen), c.stream));
+  int *cations = tmp + 2 * size_t(npen), *anions = cations + npen;
   const unsigned wb = unsigned((npen + 7) / 8);
-  k_kind_order<true><<<wb, 256, 0, c.stream>>>(npen, per, first, c.d_site_m, c.d_nbr, nullptr,
-                                               cations, nullptr, nullptr);
-  k_kind_scan<<<1, kScanThreads, 0, c.stream>>>(c.nx, c.ny, per, first, cations, tmp);
-  k_kind_order<false><<<wb, 256, 0, c.stream>>>(npen, per, first, c.d_site_m, c.d_nbr, tmp,
-                                                nullptr, c.d_order, c.d_bonds);
+  k_kind_order<true><<<wb, 256, 0, c.stream>>>(na, npen, per, c.d_atom_site, c.d_site_m, c.d_nbr,
+                                               nullptr, nullptr, cations, anions, nullptr,
+                                               nullptr);
+  k_kind_scan<<<1, kScanThreads, 0, c.stream>>>(c.nx, c.ny, cations, anions, tmp, ncations);
+  k_kind_order<false><<<wb, 256, 0, c.stream>>>(na, npen, per, c.d_atom_site, c.d_site_m, c.d_nbr,
+                                                tmp, ncations, nullptr, nullptr, c.d_order,
+                                                c.d_bonds);
   TB_CUDA(cudaGetLastError());
-  int nc = 0;
-  TB_CUDA(cudaMemcpyAsync(&nc, tmp + 2 * size_t(npen), sizeof(int), cudaMemcpyDeviceToHost,
-                          c.stream));
   TB_CUDA(cudaFreeAsync(tmp, c.stream));
-  TB_CUDA(cudaStreamSynchronize(c.stream));
-  c.ncations = nc;
   return TBGPU_OK;
 }
 
@@ -266,17 +283,13 @@ int build_topology(Ctx &c) {
   if (rc == TBGPU_OK) {
     TB_CUDA(cudaMalloc(&c.d_site_index, sizeof(int) * ns));
     TB_CUDA(cudaMalloc(&c.d_atom_site, sizeof(int) * natoms));
-    // one allocation: neighbours, bonds and work order
-    TB_CUDA(cudaMalloc(&c.d_nbr, (2 * sizeof(int4) + sizeof(int)) * natoms));
-    c.d_bonds = c.d_nbr + natoms;
-    c.d_order = reinterpret_cast<int *>(c.d_bonds + natoms);
+    TB_CUDA(cudaMalloc(&c.d_nbr, sizeof(int4) * natoms));
     TB_CUDA(cudaMalloc(&c.d_site_m, natoms));
     TB_CUDA(cudaMalloc(&c.d_surface, natoms));
     k_finalize<<<blocks, threads, 0, c.stream>>>(g, ns, flag, index, c.d_site_index,
                                                  c.d_atom_site, c.d_nbr, c.d_site_m,
                                                  c.d_surface);
     TB_CUDA(cudaGetLastError());
-    rc = build_work_order(c, index);
   }
   cudaFreeAsync(tmp, c.stream);
   cudaFreeAsync(flag, c.stream);
