@@ -122,9 +122,8 @@ constexpr int kUpdLoads = 3, kUpdBlocks = 4;
 // bet[it+1] = ||r_n||.  bet[0] is the norm of the start vector.
 template <typename VT>
 __global__ void __launch_bounds__(kRedThreads, kUpdBlocks)
-    k_update(long n2, const VT *__restrict__ w, const VT *__restrict__ rc,
-             const VT *__restrict__ rp, VT *__restrict__ rout,
-             const double *alpha, double *bet, int it, double *partial, unsigned *counter) {
+    k_update(long n2, const VT *w, const VT *rc, const VT *rp, VT *rout, const double *alpha,
+             double *bet, int it, double *partial, unsigned *counter) {
   wait_for_previous();
   const double al = alpha[it], bprev = bet[it];
   const double iq = 1.0 / bprev;

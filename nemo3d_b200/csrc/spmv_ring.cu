@@ -271,11 +271,10 @@ template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool U
 __global__ void __launch_bounds__(PAIRS * 64, 1)
     k_hx_ring(int ncat, int nan, const int *__restrict__ order, const int4 *__restrict__ bonds,
               const HT *__restrict__ onsite, const HT *__restrict__ blocks,
-              const __grid_constant__ RingCols<VT, P> A, const double *__restrict__ bet,
-              const double *__restrict__ alpha, double shift_d, double *partial,
-              unsigned int *counter, double *alpha_out, int alpha_idx,
-              const double2 *__restrict__ phase, const unsigned char *__restrict__ wrap,
-              const unsigned char *__restrict__ skip, int *status) {
+              const __grid_constant__ RingCols<VT, P> A, const double *bet, const double *alpha,
+              double shift_d, double *partial, unsigned int *counter, double *alpha_out,
+              int alpha_idx, const double2 *phase, const unsigned char *wrap,
+              const unsigned char *skip, int *status) {
   using S = RingShape<NORB, NSPIN, P, HT, VT, UPD, TA>;
   using RT = typename RealOf<VT>::T;
   constexpr int NB = S::NB, APW = S::APW, LPA = S::LPA, H = S::H, NO = S::NO;
@@ -327,7 +326,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
     const int j = first(q) + al;
     return q < tasks && live && j < last(q) ? __ldg(order + j) : -1;
   };
-  auto lane_skip = [&](int a) { return skip && a >= 0 ? int(__ldg(skip + a)) : 0; };
+  auto lane_skip = [&](int a) { return skip && a >= 0 ? int(skip[a]) : 0; };
   // a task without atoms, or whose atoms are all left out, is neither staged
   // nor computed
   auto runs = [&](int a, int left) { return __any_sync(0xffffffffu, a >= 0 && !left) != 0; };
@@ -484,7 +483,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
       iq_u = 1.0 / bp_u;
       ip_u = it > 0 ? 1.0 / bet[it - 1] : 0.0;
     }
-    auto lane_rot = [&](int a) { return PHASE && a >= 0 ? int(__ldg(wrap + a)) : 0; };
+    auto lane_rot = [&](int a) { return PHASE && a >= 0 ? int(wrap[a]) : 0; };
     auto lane_bonds = [&](int q) {  // 5-orbital models: where the blocks start
       const int j = first(q) + al;
       return S::BLKB % 16 && q < tasks && live && j < last(q) ? __ldg(bonds + j)
@@ -535,7 +534,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
           VT xn[PIPE || FLOAT ? 1 : NORB];
           if constexpr (!PIPE && !FLOAT) lds_seg(xp, xn);
           if (PHASE && rot) {
-            const double2 ph = __ldg(phase + long(max(la, 0)) * 4 + n);
+            const double2 ph = phase[long(max(la, 0)) * 4 + n];
 #pragma unroll
             for (int k = 0; k < NORB; k++) {
               const VT u = xn[k];
