@@ -47,10 +47,19 @@ int ensure_partials(Ctx &c, int nblocks) {
   return TBGPU_OK;
 }
 
-// Pinned host memory of at least `bytes` that the context keeps and grows:
-// allocating and freeing two such buffers took 1.5 to 3 ms of every solve (96
-// iterations at 45k atoms: 4.2 ms of device work).  Copies into it are
-// ordered by the context's stream.
+// Pinned host memory of at least `bytes` that the context grows and keeps from
+// solve to solve up to kPinnedKept (imax of 52,000): allocating and freeing two
+// such buffers took 1.5 to 3 ms of every solve (96 iterations at 45k atoms: 4.2
+// ms of device work).  Copies into it are ordered by the context's stream.
+constexpr size_t kPinnedKept = 4 << 20;
+
+static void pinned_release(Ctx &c) {
+  if (c.h_pinned_bytes <= kPinnedKept) return;
+  cudaFreeHost(c.h_pinned);
+  c.h_pinned = nullptr;
+  c.h_pinned_bytes = 0;
+}
+
 static int pinned_scratch(Ctx &c, size_t bytes, double **out) {
   if (bytes > c.h_pinned_bytes) {
     if (c.h_pinned) cudaFreeHost(c.h_pinned);
@@ -696,6 +705,7 @@ static int solve_t(Ctx &c, const SolveArgs &A, const double *r0_dev, double *val
     if (d_bet) cudaFreeAsync(d_bet, s);
     if (d_tmp) cudaFreeAsync(d_tmp, s);
     cudaStreamSynchronize(s);  // no return with work or copies in flight
+    pinned_release(c);
     for (auto e : spmv_ev) cudaEventDestroy(e);
     for (auto e : upd_ev) cudaEventDestroy(e);
   };
