@@ -634,8 +634,7 @@ static int solve_t(Ctx &c, const SolveArgs &A, const double *r0_dev, double *val
   c.stats.check_ms = 0.0;
   c.stats.wait_ms = 0.0;
   // eigenvector pass by regeneration (tbgpu_set_eigenvector_pass): both
-  // passes run a register-streaming kernel whose columns compute as
-  // one-column launches -- the pencil kernel when variant 6 is set and
+  // passes run a kernel whose columns compute as one-column launches -- the pencil kernel when variant 6 is set and
   // applies, else the ring kernel (variant 5)
   const bool f32_ok = !kMixed || c.ham_fp32;
   // folded-spectrum operator (tbgpu_set_fold): two products per step, plain

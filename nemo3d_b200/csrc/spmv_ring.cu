@@ -112,6 +112,11 @@ __host__ __device__ constexpr int ring_split(int norb, int p, int vector_bytes) 
   return norb == 10 && p == 1 && vector_bytes == 16 ? 2 : 1;
 }
 
+// Slots per ring: a task's own data travel with its bond kSlots.  With three,
+// fewer pairs fit (7 for 8 in double): 0.533 against 0.512 ms at 1.02M atoms,
+// float 0.315 against 0.279.
+constexpr int kSlots = 2;
+
 // Shared-memory geometry of a configuration (bytes), tasks of TA atoms at most
 template <int NORB, int NSPIN, int P, typename HT, typename VT, bool UPD, int TA>
 struct RingShape {
@@ -130,9 +135,10 @@ struct RingShape {
   // Atoms of a task whose block comes by a bulk copy, one request of the TMA
   // unit (about 17 cycles for 800 bytes, 12 for 400, as many for 200); the
   // rest come by lines through the load/store unit, which also carries the
-  // vectors.  Small blocks of single vectors leave it a quarter (2M-atom
-  // float dot 0.50 against 0.53 ms, 5-orbital dots 104 against 111 us);
-  // 800-byte blocks none (half of them by lines: 0.48 against 0.44 ms, 1.02M).
+  // vectors.  Small blocks of single vectors leave it four atoms' a task, a
+  // quarter of 16 or an eighth of 32 (2M-atom float dot 0.50 against 0.53 ms,
+  // 5-orbital dots 104 against 111 us); 800-byte blocks none (half of them by
+  // lines: 0.48 against 0.44 ms, 1.02M).
   static constexpr int BULK = BLKB >= 800 || P > 1 || APW < 16 ? APW : APW - 4;
   // a vector segment: NSPIN parts of SEG bytes
   static constexpr int SEG = NORB * int(sizeof(VT));
@@ -153,8 +159,8 @@ struct RingShape {
   static constexpr int PREV = UPD ? OWN : 0;
   static constexpr int TASK = OWN + PREV + APW * RPITCH;
   // of a warp pair: the ring, the task's own data, two barriers per slot
-  __host__ __device__ static constexpr int pair_bytes(int slots) {
-    return cdiv(slots * SLOT + TASK + 16 * slots, 128) * 128;
+  __host__ __device__ static constexpr int pair_bytes() {
+    return cdiv(kSlots * SLOT + TASK + 16 * kSlots, 128) * 128;
   }
 };
 
@@ -267,7 +273,7 @@ struct TaskMeta {
 };
 
 template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool UPD, bool PHASE,
-          int TA, int PAIRS, int SLOTS>
+          int TA, int PAIRS>
 __global__ void __launch_bounds__(PAIRS * 64, 1)
     k_hx_ring(int ncat, int nan, const int *__restrict__ order, const int4 *__restrict__ bonds,
               const HT *__restrict__ onsite, const HT *__restrict__ blocks,
@@ -286,14 +292,14 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
   const int al = live ? lane / LPA : APW - 1;          // this lane's atom of the task,
   const int h = H > 1 ? (lane % LPA) / (P * NSPIN) : 0;     // part of the orbitals,
   const int col = (lane % (P * NSPIN)) / NSPIN, sp = lane % NSPIN;  // vector and spin
-  unsigned char *wbase = smem + pair * S::pair_bytes(SLOTS);
-  unsigned char *own_p = wbase + SLOTS * S::SLOT;
+  unsigned char *wbase = smem + pair * S::pair_bytes();
+  unsigned char *own_p = wbase + kSlots * S::SLOT;
   // per slot: full (the 32 producer lanes' copies and the bulk copies landed),
   // empty (consumed)
-  const uint32_t bars = smem_addr(wbase) + S::pair_bytes(SLOTS) - 16 * SLOTS;
+  const uint32_t bars = smem_addr(wbase) + S::pair_bytes() - 16 * kSlots;
   if (warp < PAIRS && lane == 0) {
 #pragma unroll
-    for (int k = 0; k < SLOTS; k++) {
+    for (int k = 0; k < kSlots; k++) {
       mbar_init(bars + 16 * k, 33);
       mbar_init(bars + 16 * k + 8, 1);
     }
@@ -334,7 +340,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
   bool late = false;  // a bounded wait ran out
 
   if (warp >= PAIRS) {
-    // ---- producer: copies the pair's bonds in order, SLOTS ahead -----------
+    // ---- producer: copies the pair's bonds in order, kSlots ahead -----------
     constexpr bool DIRECT = P == 1 && APW <= 16;
     constexpr int U = DIRECT ? APW / 4 : 1;
     auto load_meta = [&](int q) {
@@ -359,7 +365,6 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
         cpa<S::XCH_B, true>(dst + o + (S::SP > S::SEG && o >= S::SEG ? S::SP - S::SEG : 0), src + o, ok);
       });
     };
-    static_assert(SLOTS == 2 || SLOTS == 3, "own data travel with bond SLOTS of their task");
     const uint32_t ring = smem_addr(wbase), own = smem_addr(own_p);
     uint32_t slot = 0, phase_bit = 1;  // the first pass over the slots finds them empty
     int q = place, q1 = advance(q);
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
           __syncwarp();
           // bond 0 of the task is consumed, so the task before it has left
           // the own slot: this task's own data, covered by this bond's barrier
-          if (n == SLOTS) issue_own();
+          if (n == kSlots) issue_own();
           int v[U], id[U];
 #pragma unroll
           for (int u = 0; u < U; u++) {
@@ -453,7 +458,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
               },
               [&](Src t, int s, int pc) { copy_seg(t.p, dst + APW * S::BPITCH + s * S::XP, pc, t.ok); });
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
-          if (++slot == SLOTS) {
+          if (++slot == kSlots) {
             slot = 0;
             phase_bit ^= 1;
           }
@@ -468,7 +473,7 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
     }
     cp_wait<0>();
     if (late)  // once more, bounded, for the bulk copies in flight
-      for (uint32_t k = 0; k < SLOTS; k++)
+      for (uint32_t k = 0; k < kSlots; k++)
         mbar_wait(bars + 16 * k, k < slot ? phase_bit ^ 1 : phase_bit);
   } else {
     // ---- consumer --------------------------------------------------------------
@@ -687,13 +692,13 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
           if (BULK_OUT && n == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();  // every lane has read the slot
           if (lane == 0) mbar_arrive(full + 8);
-          if (++slot == SLOTS) {
+          if (++slot == kSlots) {
             slot = 0;
             phase_bit ^= 1;
           }
         }
         if (late) break;
-        // own data: copied before bond SLOTS of the task and so covered by its
+        // own data: copied before bond kSlots of the task and so covered by its
         // full barrier
         const VT *xo_p = reinterpret_cast<const VT *>(own_p + seg);
         const VT *ot_p = reinterpret_cast<const VT *>(own_p + (al * P + col) * S::XP + (NSPIN - 1 - sp) * S::SP);
@@ -818,17 +823,13 @@ __global__ void __launch_bounds__(PAIRS * 64, 1)
 }
 
 constexpr int kMaxSmem = 227 * 1024;
-// Slots per ring.  With three, fewer pairs fit: 0.567 (6 pairs) against 0.541
-// ms at 1.02M atoms, double.
-constexpr int kSlots = 2;
-
 // Warp pairs per SM: as many as shared memory holds, at most 12; the
 // 10-orbital double products take at most eight, which leaves them the 128
 // registers a thread they need (nine: 0.63 against 0.53 ms at 1.02M atoms,
 // block of 4 at 381k 0.73 against 0.55).
 template <class S>
 constexpr int ring_pairs(bool wide) {
-  const int w = kMaxSmem / S::pair_bytes(kSlots), most = wide ? 8 : 12;
+  const int w = kMaxSmem / S::pair_bytes(), most = wide ? 8 : 12;
   return w > most ? most : w;
 }
 
@@ -846,10 +847,10 @@ template <int NORB, int NSPIN, int P, typename HT, typename VT, bool DOT, bool U
           int TA = 32>
 int run_ring(Ctx &c, const RingCols<VT, P> &A, RingLaunch L, cudaStream_t s) {
   using S = RingShape<NORB, NSPIN, P, HT, VT, UPD, TA>;
-  constexpr int SLOTS = kSlots, PAIRS = ring_pairs<S>(NORB == 10 && sizeof(VT) == 16);
-  constexpr int smem = PAIRS * S::pair_bytes(SLOTS);
+  constexpr int PAIRS = ring_pairs<S>(NORB == 10 && sizeof(VT) == 16);
+  constexpr int smem = PAIRS * S::pair_bytes();
   static_assert(PAIRS >= 1, "a task does not fit shared memory");
-  const auto kernel = k_hx_ring<NORB, NSPIN, P, HT, VT, DOT, UPD, PHASE, TA, PAIRS, SLOTS>;
+  const auto kernel = k_hx_ring<NORB, NSPIN, P, HT, VT, DOT, UPD, PHASE, TA, PAIRS>;
   static std::atomic<unsigned long long> attr_done{0};
   if (ensure_smem_attr(attr_done, c.device, kernel, smem)) return TBGPU_E_CUDA;
   const int ncat = int(c.ncations), nan = int(c.natoms - c.ncations);

@@ -13,10 +13,6 @@ namespace stage {
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ void cp16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
-               : "memory");
-}
 // 16-byte copy that reads `bytes` (16 or 0) from global memory and fills the
 // rest of the chunk with zeros: a missing neighbour costs no branch
 __device__ __forceinline__ void cp16z(void *dst, const void *src, int bytes) {
