@@ -220,7 +220,7 @@ int tbgpu_build_hamiltonian(tbgpu_ctx *ctx) {
     if (rc == TBGPU_OK) c.topo_built = true;
   }
   if (rc == TBGPU_OK) rc = assemble(c);
-  if (rc == TBGPU_OK) rc = ensure_partials(c, int(c.natoms / 8 + 65536));
+  if (rc == TBGPU_OK) rc = ensure_partials(c, partials_of_build(c));
   cudaEventRecord(e1, c.stream);
   if (cudaStreamSynchronize(c.stream) != cudaSuccess && rc == TBGPU_OK) rc = set_error(TBGPU_E_CUDA);
   int st[2] = {0, 0};  // status, cations

@@ -277,6 +277,8 @@ int launch_spmv_scratch(Ctx &c, const double *x, double *y, double shift, double
                         unsigned int *counter, int cap, double *dot_out, cudaStream_t s);
 // lanczos.cu
 int ensure_partials(Ctx &c, int nblocks);
+// block partials that a build provides for
+inline int partials_of_build(const Ctx &c) { return int(c.natoms / 8 + 65536); }
 // y = F x (the folded operator) on double vectors in the reference's order
 int fold_product(Ctx &c, const double *x, double *y, double *tmp, cudaStream_t s);
 struct SolveArgs {

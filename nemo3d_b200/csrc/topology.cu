@@ -8,6 +8,8 @@
 //   FindSurfaceAtoms (bit 0, isOnSurface) nemo3d/src/base/geo_struct.c:1374-1463
 // Atoms are numbered in site order (cell-major, k fastest, then in-cell site),
 // which is the reference's vector layout.
+#include <algorithm>
+
 #include <cub/block/block_scan.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -233,14 +235,17 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 
 // into room (natoms * kOrderBytes, 16-byte aligned) behind the stored blocks;
-// *ncations (device) receives the count of cations
+// *ncations (device) receives the count of cations.  The counts per pencil are
+// kept in the reduction scratch meanwhile: a stream-ordered allocation would
+// map memory again, which the pool has given back in the waits before.
 int build_work_order(Ctx &c, void *room, int *ncations) {
   const int na = int(c.natoms), npen = c.nx * c.ny;
   const long per = long(c.nz) * 8;
   c.d_bonds = static_cast<int4 *>(room);
   c.d_order = reinterpret_cast<int *>(c.d_bonds + na);
-  int *tmp = nullptr;  // at[2 npen], cations[npen], anions[npen]
-  TB_CUDA(cudaMallocAsync(&tmp, sizeof(int) * 4 * size_t(npen), c.stream));
+  const int rc = ensure_partials(c, std::max(partials_of_build(c), 2 * npen));
+  if (rc) return rc;
+  int *tmp = reinterpret_cast<int *>(c.d_partial);  // at[2 npen], cations[npen], anions[npen]
   int *cations = tmp + 2 * size_t(npen), *anions = cations + npen;
   const unsigned wb = unsigned((npen + 7) / 8);
   k_kind_order<true><<<wb, 256, 0, c.stream>>>(na, npen, per, c.d_atom_site, c.d_site_m, c.d_nbr,
@@ -251,7 +256,6 @@ int build_work_order(Ctx &c, void *room, int *ncations) {
                                                 tmp, ncations, nullptr, nullptr, c.d_order,
                                                 c.d_bonds);
   TB_CUDA(cudaGetLastError());
-  TB_CUDA(cudaFreeAsync(tmp, c.stream));
   return TBGPU_OK;
 }
 

@@ -93,3 +93,23 @@ def _abs_row_sum(o):
     blk = np.abs(o.blocks).reshape(-1, o.norb, o.norb)
     ons = np.abs(o.onsite).reshape(o.natoms, o.nb, -1).sum(-1).max()
     return ons + 4 * max(blk.sum(1).max(), blk.sum(2).max())
+
+
+@pytest.mark.parametrize("model", ["sp3s*", "sp3d5s*_so"])
+def test_few_atoms_in_a_wide_flat_grid(model):
+    """90,000 pencils, atoms in 60 of them at two corners: the work order's
+    counts per pencil need more scratch than the products' reductions."""
+    from nemo3d_b200.tbgpu import Hamiltonian
+    st = _alloy((300, 300, 1))
+    keep = np.zeros(st.types.shape, bool)
+    keep[:6, :5] = keep[-5:, -6:] = True
+    st.types[~keep] = 0
+    st = workloads.Structure(300, 300, 1, st.lattice, (False,) * 3, st.types, st.dsp)
+    fam = "sps" if model.startswith("sp3s*") else "spds"
+    mats = [materials.MATERIALS["GaAs_" + fam], materials.MATERIALS["InAs_" + fam]]
+    g = Hamiltonian(st, model, mats)
+    o = oracle.OracleHamiltonian(st, *materials.BAND_MODELS[model], mats)
+    assert 300 < g.natoms == o.natoms <= 480
+    scale = max(np.abs(o.onsite).max(), np.abs(o.blocks).max())
+    x = np.random.default_rng(6).uniform(-1, 1, 2 * g.n)
+    assert np.abs(g.matvect_mult(x, 0.7) - o.hx(x, 0.7)).max() <= 45e-12 * scale
