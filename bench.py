@@ -63,9 +63,9 @@ METRIC = "s to 8 band-edge eigenpairs at <=1e-6 eV vs plain FP64 GPU Lanczos; Sp
 # x read once, y written once): FP64 1864 + 640, complex-float 936 + 320.
 BYTES_PER_ATOM = {64: 2504, 32: 1256}
 # DRAM bytes per atom of one H*x launch, measured with ncu (dram__bytes_read
-# + dram__bytes_write, one launch, cold L2) and scaled by atoms: the ring
-# kernel at 1.99M atoms (float) and at 1.02M (FP64).
-NCU_TRAFFIC_PER_ATOM = {32: 1377, 64: 2610}
+# + dram__bytes_write, one launch) and scaled by atoms: the ring kernel at
+# 1.99M atoms (float) and at 1.02M (FP64), profiles/k_hx_ring_forms_ncu.md.
+NCU_TRAFFIC_PER_ATOM = {32: 1331, 64: 2607}
 # one complex vector per atom (20 entries: FP64 320 B, complex float 160 B) and
 # the stored blocks + on-site records + neighbour columns per atom (B_H)
 VEC_PER_ATOM = {64: 320, 32: 160}
